@@ -41,6 +41,7 @@ LIB_SOURCES = [
     "csrc/server.cpp",
     "csrc/capi.cpp",
     "csrc/plan.cpp",
+    "csrc/key_product.cu",
     "csrc/decrypt.cu",
     "csrc/encrypt.cu",
     "csrc/host/idash_host.cpp",

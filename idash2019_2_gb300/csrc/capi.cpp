@@ -6,6 +6,7 @@
 #include <thread>
 
 #include "capi_internal.hpp"
+#include "key_product.cuh"
 
 using namespace idash;
 
@@ -571,6 +572,7 @@ idash_status idash_open(idash_ctx **out, int device) {
     }
     if (s == IDASH_OK) s = ctx->check_cuda(configure_window_kernels(ctx->smem_optin), "configure kernels");
     if (s == IDASH_OK) s = ctx->check_cuda(configure_tc_kernel(ctx->smem_optin), "configure tensor-core kernel");
+    if (s == IDASH_OK) s = ctx->check_cuda(configure_key_product(), "configure key product kernels");
     if (s == IDASH_OK) s = ctx->check_cuda(cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking), "cudaStreamCreate");
     if (s == IDASH_OK) s = ctx->check_cuda(cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking), "cudaStreamCreate");
     if (s == IDASH_OK) s = ctx->check_cuda(cudaEventCreateWithFlags(&ctx->join_in, cudaEventDisableTiming), "cudaEventCreate");

@@ -4,16 +4,15 @@
 // Z/2^32 with the integer key s) and reads its coefficients
 // [0, NUM_SAMPLES) as t32tod(phase[j]) = phase[j] / 2^32, stored as float.
 //
-// The product is exact: only the key's nonzero coefficients are visited (a
-// TFHE key is binary, so about N/2 of them), and each of the NUM_SAMPLES
-// coefficients is a sum of N/2 words mod 2^32.  The float conversion
+// The product is exact: on the tensor cores for binary keys (key_product.cu),
+// else as a sum over the key's nonzero coefficients.  The float conversion
 // float(phase / 2^32) equals float(phase) * 2^-32 exactly (scaling by a power
 // of two commutes with round-to-nearest for these magnitudes).
 #include <algorithm>
 
 #include "capi_internal.hpp"
 #include "common.cuh"
-#include "negacyclic.cuh"
+#include "key_product.cuh"
 
 namespace idash {
 namespace {
@@ -75,46 +74,6 @@ __global__ void __launch_bounds__(kDecryptThreads) k_decrypt_phase(const uint8_t
     }
 }
 
-// Binary keys, N a multiple of 32: the register-windowed product of
-// negacyclic.cuh, kNegCols consecutive coefficients per thread, kRowsPerCta
-// rows per CTA, each with its own padded extension.  Measured on the
-// 242,646 x 1,000 decryption: 8 columns per thread 8.4 ms, 16 columns 7.0 ms,
-// 32 columns 8.1 ms (k_decrypt_phase: 15.2 ms); testing the key bits in
-// pairs (one three-input add for two set bits) was slower at every width.
-template <uint32_t kRowThreads>
-__global__ void __launch_bounds__(kDecryptThreads) k_decrypt_binary(const uint8_t *in, uint64_t in_stride, uint32_t N,
-                                                                    uint32_t num_samples, const uint32_t *key_idx,
-                                                                    uint32_t n_nz, uint64_t n_rows, float *out) {
-    constexpr uint32_t kRowsPerCta = kDecryptThreads / kRowThreads;
-    extern __shared__ __align__(16) uint32_t sh[];
-    uint32_t *key_mask = sh;
-    uint32_t *ext_all = sh + neg_mask_words(N);  // kRowsPerCta padded extensions
-    neg_build_mask(key_mask, N, key_idx, n_nz);
-    const uint32_t sub = threadIdx.x / kRowThreads, x = threadIdx.x % kRowThreads;
-    const uint32_t j0 = kNegCols * x;
-    const uint32_t ext_words = neg_ext_words(N);
-    for (uint64_t row0 = uint64_t(blockIdx.x) * kRowsPerCta; row0 < n_rows; row0 += uint64_t(gridDim.x) * kRowsPerCta) {
-        __syncthreads();  // the previous rows are done with ext (and the key mask is complete)
-        for (uint32_t t = threadIdx.x; t < kRowsPerCta * N; t += blockDim.x) {
-            const uint32_t s = t / N, k = t % N;
-            if (row0 + s >= n_rows) break;
-            neg_store(ext_all + s * ext_words, N, k, reinterpret_cast<const uint32_t *>(in + (row0 + s) * in_stride)[k]);
-        }
-        __syncthreads();
-        const uint64_t row = row0 + sub;
-        if (row >= n_rows || j0 >= num_samples) continue;
-        uint32_t acc[kNegCols];
-        neg_product(ext_all + sub * ext_words, N, j0, key_mask, acc);
-        const uint32_t *b = reinterpret_cast<const uint32_t *>(in + row * in_stride) + N;
-        float *o = out + row * num_samples;
-#pragma unroll
-        for (uint32_t r = 0; r < kNegCols; ++r) {
-            const uint32_t j = j0 + r;
-            if (j < num_samples) o[j] = __int2float_rn(int32_t(b[j] - acc[r])) * 0x1p-32f;
-        }
-    }
-}
-
 }  // namespace
 }  // namespace idash
 
@@ -131,38 +90,27 @@ extern "C" idash_status idash_decrypt_trlwe_device(idash_ctx *ctx, const int32_t
         return ctx->fail(IDASH_ERR_INVALID_ARGUMENT, "idash_decrypt_trlwe_device: bad row layout");
     if (n_rows == 0) return IDASH_OK;
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+    const uint8_t *in = static_cast<const uint8_t *>(d_in) + in_layout->payload_offset;
+    // Binary keys (TFHE's) of a size the product kernel takes: tensor cores,
+    // the key in the launch parameters.  242,646 rows x 1,000 scores at
+    // N = 1024: 7.00 ms with the product on CUDA cores, 1.67 ms
+    // here.
+    KeyProductArgs kp{};
+    if (key_product_supported(N) && key_bits(key, N, &kp.key)) {
+        kp.rows = const_cast<uint8_t *>(in);  // read only when scores are asked for
+        kp.stride = in_layout->row_stride;
+        kp.n_rows = n_rows;
+        kp.N = N;
+        kp.n_coef = num_samples;
+        kp.scores = d_out;
+        kp.err = ctx->d_err;
+        const idash_status r = ctx->check_cuda(launch_key_product(kp, ctx->sm_count, s), "k_key_product launch");
+        if (r == IDASH_OK) ctx->stats.kernel_launches++;
+        return r;
+    }
     StagedKey k;
     idash_status st = ctx->check_cuda(stage_key(key, N, s, &k), "key upload");
     if (st != IDASH_OK) return st;
-    const uint8_t *in = static_cast<const uint8_t *>(d_in) + in_layout->payload_offset;
-    if (k.binary && N % 32 == 0) {
-        // threads per row: kNegCols coefficients each, rounded up to whole warps
-        const uint32_t need = (num_samples + kNegCols - 1) / kNegCols;
-        const uint32_t row_threads = need <= 32 ? 32 : need <= 64 ? 64 : 128;  // need <= 2048 / kNegCols
-        const uint32_t rows_per_cta = kDecryptThreads / row_threads;
-        const size_t smem = (size_t(neg_mask_words(N)) + size_t(rows_per_cta) * neg_ext_words(N)) * 4;
-        auto launch = [&](auto kernel) {
-            // up to 8 rows of 2.25N words (144 KiB at N = 2048): above the default 48 KiB
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kDecryptThreads, smem) != cudaSuccess ||
-                per_sm < 1)
-                per_sm = 1;
-            const uint64_t ctas = (n_rows + rows_per_cta - 1) / rows_per_cta;
-            const uint32_t blocks = uint32_t(std::min<uint64_t>(ctas, uint64_t(ctx->sm_count) * per_sm));
-            kernel<<<blocks, kDecryptThreads, smem, s>>>(in, in_layout->row_stride, N, num_samples, k.idx, k.n_nz,
-                                                         n_rows, d_out);
-            return cudaGetLastError();
-        };
-        const cudaError_t le = row_threads == 32   ? launch(k_decrypt_binary<32>)
-                               : row_threads == 64 ? launch(k_decrypt_binary<64>)
-                                                   : launch(k_decrypt_binary<128>);
-        st = ctx->check_cuda(le, "k_decrypt_binary launch");
-        release_key(&k, s);
-        if (st == IDASH_OK) ctx->stats.kernel_launches++;
-        return st;
-    }
     const size_t smem = size_t(2) * N * 4 + size_t(k.n_nz) * (k.binary ? 4 : 8);
     const uint32_t blocks = uint32_t(std::min<uint64_t>(n_rows, uint64_t(ctx->sm_count) * 8));
     if (k.binary)

@@ -8,13 +8,14 @@
 // Randomness is counter-based (splitmix64 over seed, stream, index), so rows
 // are independent of the launch shape.  Streams: 21 mask words, 22 noise.
 // Noise: Box-Muller on two 24-bit uniforms, scaled by alpha * 2^32 and
-// truncated toward zero as dtot32 truncates.  The product a*s visits the
-// key's nonzero coefficients only (exact mod 2^32).
+// truncated toward zero as dtot32 truncates.  The product a*s is exact mod
+// 2^32: on the tensor cores for binary keys (key_product.cu), else a sum over
+// the key's nonzero coefficients.
 #include <algorithm>
 
 #include "capi_internal.hpp"
 #include "common.cuh"
-#include "negacyclic.cuh"
+#include "key_product.cuh"
 
 namespace idash {
 namespace {
@@ -72,6 +73,15 @@ __device__ __forceinline__ void enc_finish(const EncArgs &a, uint64_t r, uint32_
     if (a.noise) a.noise[r * a.N + j] = e_j;
 }
 
+// Header and variance of row r's record.
+__device__ __forceinline__ void enc_record(const EncArgs &a, uint64_t r, uint8_t *rec) {
+    if (a.hdr_off >= 0) {
+        *reinterpret_cast<uint32_t *>(rec + a.hdr_off) = a.row_index ? a.row_index[r] : uint32_t(r);
+        *reinterpret_cast<int32_t *>(rec + a.hdr_off + 4) = a.tag;
+    }
+    if (a.var_off >= 0) *reinterpret_cast<double *>(rec + a.var_off) = a.variance;
+}
+
 // One CTA per row (grid-stride).  Shared memory: ext[2N], the negacyclic
 // extension of the fresh mask (ext[N + t] = a[t], ext[t] = -a[t]), then the
 // key's nonzero positions and values.  Thread t owns coefficients t + 256c.
@@ -118,58 +128,23 @@ __global__ void __launch_bounds__(kEncThreads) k_encrypt_rows(const EncArgs a) {
                 enc_finish(a, r, j, acc[c], body);
             }
         }
-        if (threadIdx.x == 0) {
-            if (a.hdr_off >= 0) {
-                *reinterpret_cast<uint32_t *>(rec + a.hdr_off) = a.row_index ? a.row_index[r] : uint32_t(r);
-                *reinterpret_cast<int32_t *>(rec + a.hdr_off + 4) = a.tag;
-            }
-            if (a.var_off >= 0) *reinterpret_cast<double *>(rec + a.var_off) = a.variance;
-        }
+        if (threadIdx.x == 0) enc_record(a, r, rec);
     }
 }
 
-// Binary keys, N a multiple of 32: the register-windowed product of
-// negacyclic.cuh, kNegCols consecutive coefficients per thread, kRowsPerCta
-// rows per CTA, each with its own padded extension of its fresh mask.
-template <uint32_t kRowThreads>
-__global__ void __launch_bounds__(kEncThreads) k_encrypt_binary(const EncArgs a) {
-    constexpr uint32_t kRowsPerCta = kEncThreads / kRowThreads;
-    extern __shared__ __align__(16) uint32_t sh[];
-    const uint32_t N = a.N;
-    uint32_t *key_mask = sh;
-    uint32_t *ext_all = sh + neg_mask_words(N);  // kRowsPerCta padded extensions
-    neg_build_mask(key_mask, N, a.key_idx, a.n_nz);
-    const uint32_t sub = threadIdx.x / kRowThreads, x = threadIdx.x % kRowThreads;
-    const uint32_t j0 = kNegCols * x;
-    const uint32_t ext_words = neg_ext_words(N);
-    for (uint64_t r0 = uint64_t(blockIdx.x) * kRowsPerCta; r0 < a.n_rows; r0 += uint64_t(gridDim.x) * kRowsPerCta) {
-        __syncthreads();  // the previous rows are done with ext (and the key mask is complete)
-        for (uint32_t t = threadIdx.x; t < kRowsPerCta * N; t += blockDim.x) {
-            const uint32_t s = t / N, k = t % N;
-            const uint64_t r = r0 + s;
-            if (r >= a.n_rows) break;
-            const uint32_t v = enc_hash(a.key_a, r * N + k);
-            neg_store(ext_all + s * ext_words, N, k, v);
-            const uint64_t orow = a.row_out ? a.row_out[r] : r;
-            reinterpret_cast<uint32_t *>(a.out + orow * a.out_stride + a.payload_off)[k] = v;
+// Rows without their product: fresh masks, and bodies of noise and message
+// alone; launch_key_product then adds a*s (binary keys).  One CTA per row
+// (grid-stride): every coefficient is independent, so the hashes and the
+// Box-Muller arithmetic (what bounds this kernel) run at full occupancy.
+__global__ void __launch_bounds__(kEncThreads) k_encrypt_fresh(const EncArgs a) {
+    for (uint64_t r = blockIdx.x; r < a.n_rows; r += gridDim.x) {
+        uint8_t *rec = a.out + (a.row_out ? uint64_t(a.row_out[r]) : r) * a.out_stride;
+        uint32_t *mask = reinterpret_cast<uint32_t *>(rec + a.payload_off);
+        for (uint32_t j = threadIdx.x; j < a.N; j += kEncThreads) {
+            mask[j] = enc_hash(a.key_a, r * a.N + j);
+            enc_finish(a, r, j, 0u, mask + a.N);
         }
-        __syncthreads();
-        const uint64_t r = r0 + sub;
-        if (r >= a.n_rows || j0 >= N) continue;
-        uint32_t acc[kNegCols];
-        neg_product(ext_all + sub * ext_words, N, j0, key_mask, acc);
-        const uint64_t orow = a.row_out ? a.row_out[r] : r;
-        uint8_t *rec = a.out + orow * a.out_stride;
-        uint32_t *body = reinterpret_cast<uint32_t *>(rec + a.payload_off) + N;
-#pragma unroll 4
-        for (uint32_t q = 0; q < kNegCols; ++q) enc_finish(a, r, j0 + q, acc[q], body);
-        if (x == 0) {
-            if (a.hdr_off >= 0) {
-                *reinterpret_cast<uint32_t *>(rec + a.hdr_off) = a.row_index ? a.row_index[r] : uint32_t(r);
-                *reinterpret_cast<int32_t *>(rec + a.hdr_off + 4) = a.tag;
-            }
-            if (a.var_off >= 0) *reinterpret_cast<double *>(rec + a.var_off) = a.variance;
-        }
+        if (threadIdx.x == 0) enc_record(a, r, rec);
     }
 }
 
@@ -195,9 +170,6 @@ extern "C" idash_status idash_encrypt_trlwe_device(idash_ctx *ctx, const idash_e
         return ctx->fail(IDASH_ERR_INVALID_ARGUMENT, "idash_encrypt_trlwe_device: bad buffers or layout");
     if (n_rows == 0) return IDASH_OK;
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-    StagedKey k;
-    idash_status st = ctx->check_cuda(stage_key(key, p->N, s, &k), "key upload");
-    if (st != IDASH_OK) return st;
     EncArgs a{};
     a.N = p->N;
     a.num_samples = p->num_samples;
@@ -211,9 +183,6 @@ extern "C" idash_status idash_encrypt_trlwe_device(idash_ctx *ctx, const idash_e
     a.key_a = mix64(seed + mix64(21));
     a.key_e = mix64(seed + mix64(22));
     a.n_rows = n_rows;
-    a.key_idx = k.idx;
-    a.key_val = k.val;
-    a.n_nz = k.n_nz;
     a.slot_src = d_slot_src;
     a.geno = d_geno;
     a.geno_stride = geno_stride;
@@ -225,33 +194,30 @@ extern "C" idash_status idash_encrypt_trlwe_device(idash_ctx *ctx, const idash_e
     a.var_off = out_layout->variance_offset;
     a.hdr_off = out_layout->header_offset;
     a.noise = d_noise;
-    if (k.binary && p->N % 32 == 0) {
-        // threads per row: kNegCols coefficients each, rounded up to whole warps
-        const uint32_t need = p->N / kNegCols;
-        const uint32_t row_threads = need <= 32 ? 32 : need <= 64 ? 64 : 128;  // N <= 2048
-        const uint32_t rows_per_cta = kEncThreads / row_threads;
-        const size_t smem = (size_t(neg_mask_words(p->N)) + size_t(rows_per_cta) * neg_ext_words(p->N)) * 4;
-        auto launch = [&](auto kernel) {
-            // up to 8 rows of 2.25N words (144 KiB at N = 2048): above the default 48 KiB
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-            if (e != cudaSuccess) return e;
-            int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kEncThreads, smem) != cudaSuccess ||
-                per_sm < 1)
-                per_sm = 1;
-            const uint64_t ctas = (n_rows + rows_per_cta - 1) / rows_per_cta;
-            const uint32_t blocks = uint32_t(std::min<uint64_t>(ctas, uint64_t(ctx->sm_count) * per_sm));
-            kernel<<<blocks, kEncThreads, smem, s>>>(a);
-            return cudaGetLastError();
-        };
-        const cudaError_t le = row_threads == 32   ? launch(k_encrypt_binary<32>)
-                               : row_threads == 64 ? launch(k_encrypt_binary<64>)
-                                                   : launch(k_encrypt_binary<128>);
-        st = ctx->check_cuda(le, "k_encrypt_binary launch");
-        release_key(&k, s);
-        if (st == IDASH_OK) ctx->stats.kernel_launches++;
-        return st;
+    // Binary keys (TFHE's) of a size the product kernel takes: fresh rows, then
+    // a*s on the tensor cores, the key in the launch parameters.  48,552 rows
+    // at N = 1024: 2.49 ms with the product on CUDA cores, 0.71 ms here.
+    KeyProductArgs kp{};
+    if (key_product_supported(p->N) && key_bits(key, p->N, &kp.key)) {
+        kp.rows = a.out + a.payload_off;
+        kp.stride = a.out_stride;
+        kp.row_map = d_row_out;
+        kp.n_rows = n_rows;
+        kp.N = kp.n_coef = p->N;
+        kp.err = ctx->d_err;
+        const uint32_t blocks = uint32_t(std::min<uint64_t>(n_rows, uint64_t(ctx->sm_count) * 8));
+        k_encrypt_fresh<<<blocks, kEncThreads, 0, s>>>(a);
+        idash_status r = ctx->check_cuda(cudaGetLastError(), "k_encrypt_fresh launch");
+        if (r == IDASH_OK) r = ctx->check_cuda(launch_key_product(kp, ctx->sm_count, s), "k_key_product launch");
+        if (r == IDASH_OK) ctx->stats.kernel_launches += 2;
+        return r;
     }
+    StagedKey k;
+    idash_status st = ctx->check_cuda(stage_key(key, p->N, s, &k), "key upload");
+    if (st != IDASH_OK) return st;
+    a.key_idx = k.idx;
+    a.key_val = k.val;
+    a.n_nz = k.n_nz;
     const size_t smem = size_t(2) * p->N * 4 + size_t(a.n_nz) * 8;
     const uint32_t blocks = uint32_t(std::min<uint64_t>(n_rows, uint64_t(ctx->sm_count) * 8));
     if (k.binary)

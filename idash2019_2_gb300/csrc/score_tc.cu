@@ -49,6 +49,7 @@
 
 #include "common.cuh"
 #include "score_kernels.cuh"
+#include "tcgen05.cuh"
 
 namespace idash {
 
@@ -68,6 +69,7 @@ constexpr uint32_t kHeader = 1024;
 constexpr uint32_t kThreads = 320;
 constexpr uint32_t kProducerWarp = 4, kMmaWarp = 5, kConvWarp0 = 6;
 constexpr uint32_t kTmemCols = 512;                     // 2 stages x 4 accumulators x 64 columns
+constexpr uint32_t kIdesc = umma_idesc_f16(kM, kN);
 constexpr uint32_t kMagic = 0x4B400000u;                // bits of 1.5 * 2^23
 constexpr uint32_t kMagicSum = kMagic + (kMagic << 8) + (kMagic << 16) + (kMagic << 24);
 // one CTA per SM, so the CTA owns all of TMEM
@@ -88,68 +90,6 @@ __device__ __forceinline__ void expect_tx(uint64_t *bar, uint32_t bytes) {
                  : "memory");
 }
 
-__device__ __forceinline__ bool aborted(const TcBars &sh) {
-    return *reinterpret_cast<const volatile uint32_t *>(&sh.abort) != 0;
-}
-
-// Bounded wait that also ends when another role raised the abort flag.
-__device__ __forceinline__ bool tc_wait(TcBars &sh, uint64_t *bar, uint32_t parity, uint32_t *err) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait_sleep(bar, parity, 20000u)) {
-        if (aborted(sh)) return false;
-        if (clock64() - t0 > kWaitLimitCycles) {
-            report_error(err, kDevTimeout);
-            *reinterpret_cast<volatile uint32_t *>(&sh.abort) = 1u;
-            return false;
-        }
-    }
-    return true;
-}
-
-// Lane 0 waits, the warp follows its verdict.
-__device__ __forceinline__ bool warp_wait(TcBars &sh, uint64_t *bar, uint32_t parity, uint32_t *err, uint32_t lane) {
-    uint32_t ok = 1;
-    if (lane == 0) ok = tc_wait(sh, bar, parity, err) ? 1u : 0u;
-    return __shfl_sync(0xFFFFFFFFu, ok, 0) != 0;
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// Shared-memory matrix descriptor, no swizzle: start address, LBO = bytes
-// between core matrices along K, SBO = bytes between 8-row groups.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return uint64_t((saddr & 0x3FFFFu) >> 4) | (uint64_t((lbo >> 4) & 0x3FFFu) << 16) |
-           (uint64_t((sbo >> 4) & 0x3FFFu) << 32) | (uint64_t(1) << 46);
-}
-
-// D (fp32, TMEM) (+)= A (fp16, K-major) * B (fp16, K-major), M = 128, N = 64.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
-    constexpr uint32_t idesc = (1u << 4) | ((kN >> 3) << 17) | ((kM >> 4) << 24);
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(addr)
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
 // 2D tensor copy of the box at (x = column, y = row) into shared memory,
 // completed on `bar` as transaction bytes.  x * 4 is a multiple of 16.
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int32_t x, int32_t y, uint64_t *bar) {
@@ -164,11 +104,6 @@ __device__ __forceinline__ uint4 lds_v4p(const uint32_t *p) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr(p)));
     return v;
-}
-
-__device__ __forceinline__ void sts_v4(uint32_t *p, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(smem_addr(p)), "r"(x), "r"(y), "r"(z), "r"(w)
-                 : "memory");
 }
 
 // fp16x2 bits {lo: v_lo - 128, hi: v_hi - 128} from r = [v_lo, 0x64, v_hi, 0x64]
@@ -222,10 +157,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
         fence_mbar_init();
     }
     if (warp == kMmaWarp) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)),
-                     "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tmem_alloc(&sh.tmem_base, kTmemCols);
     }
     tc_fence_before();
     __syncthreads();
@@ -238,7 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
         bool ok = true;
         for (uint32_t u = blockIdx.x, uc = 0; ok && u < a.n_units; u += gridDim.x, ++uc) {
             const Unit x = unit_of(a, u);
-            if (uc > 0 && !(ok = warp_wait(sh, &sh.a_empty, (uc - 1) & 1u, a.err, lane))) break;
+            if (uc > 0 && !(ok = tc_warp_wait(&sh.abort, &sh.a_empty, (uc - 1) & 1u, a.err, lane))) break;
             if (lane == 0) {
                 const uint32_t bytes = 4u * kM * x.k_pad;  // tc_a_bytes(k_pad): two fp16 digit planes
                 fence_proxy_async_smem();
@@ -253,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
                 for (uint32_t c = 0; c < x.n_chunks; ++c) {
                     const uint32_t st = rc % kRawStages;
                     if (rc >= kRawStages &&
-                        !(ok = warp_wait(sh, &sh.raw_empty[st], ((rc / kRawStages) - 1) & 1u, a.err, lane)))
+                        !(ok = tc_warp_wait(&sh.abort, &sh.raw_empty[st], ((rc / kRawStages) - 1) & 1u, a.err, lane)))
                         break;
                     if (lane == 0) fence_proxy_async_smem();
                     __syncwarp();
@@ -311,9 +243,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
             for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl) {
                 for (uint32_t c = 0; c < x.n_chunks; ++c, ++rc) {
                     const uint32_t st = rc % kRawStages, dg = rc % kDigStages;
-                    if (!(ok = warp_wait(sh, &sh.raw_full[st], (rc / kRawStages) & 1u, a.err, lane))) break;
+                    if (!(ok = tc_warp_wait(&sh.abort, &sh.raw_full[st], (rc / kRawStages) & 1u, a.err, lane))) break;
                     if (rc >= kDigStages &&
-                        !(ok = warp_wait(sh, &sh.dig_empty[dg], ((rc / kDigStages) - 1) & 1u, a.err, lane)))
+                        !(ok = tc_warp_wait(&sh.abort, &sh.dig_empty[dg], ((rc / kDigStages) - 1) & 1u, a.err, lane)))
                         break;
                     const uint32_t rows = min(kChunk, x.k_pad - c * kChunk);
                     if (2 * kp < rows) {
@@ -350,18 +282,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
             const uint32_t a_base = smem_addr(smA), d_base = smem_addr(dig);
             for (uint32_t u = blockIdx.x, uc = 0; ok && u < a.n_units; u += gridDim.x, ++uc) {
                 const Unit x = unit_of(a, u);
-                if (!(ok = tc_wait(sh, &sh.a_full, uc & 1u, a.err))) break;
+                if (!(ok = tc_wait(&sh.abort, &sh.a_full, uc & 1u, a.err))) break;
                 const uint32_t a_plane = x.k_pad * 256;  // bytes per coefficient digit plane
                 for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl, ++tcount) {
                     const uint32_t acc = tcount % kAccStages;
                     if (tcount >= kAccStages &&
-                        !(ok = tc_wait(sh, &sh.acc_empty[acc], ((tcount / kAccStages) - 1) & 1u, a.err)))
+                        !(ok = tc_wait(&sh.abort, &sh.acc_empty[acc], ((tcount / kAccStages) - 1) & 1u, a.err)))
                         break;
                     tc_fence_after();
                     const uint32_t d0 = tmem + acc * 256;
                     for (uint32_t c = 0; c < x.n_chunks; ++c, ++rc) {
                         const uint32_t dg = rc % kDigStages;
-                        if (!(ok = tc_wait(sh, &sh.dig_full[dg], (rc / kDigStages) & 1u, a.err))) break;
+                        if (!(ok = tc_wait(&sh.abort, &sh.dig_full[dg], (rc / kDigStages) & 1u, a.err))) break;
                         tc_fence_after();
                         const uint32_t steps = min(kChunk, x.k_pad - c * kChunk) / 16;
                         const uint32_t b_base = d_base + dg * kDigStageBytes;
@@ -373,13 +305,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
                             const uint64_t b1 = umma_desc(b_base + kPlaneBytes + j * 2048, 1024, 128);
                             const uint64_t b2 = umma_desc(b_base + 2 * kPlaneBytes + j * 2048, 1024, 128);
                             const uint64_t b3 = umma_desc(b_base + 3 * kPlaneBytes + j * 2048, 1024, 128);
-                            umma_f16(d0, a0, b0, on);
-                            umma_f16(d0 + 64, a0, b1, on);
-                            umma_f16(d0 + 64, a1, b0, 1u);
-                            umma_f16(d0 + 128, a0, b2, on);
-                            umma_f16(d0 + 128, a1, b1, 1u);
-                            umma_f16(d0 + 192, a0, b3, on);
-                            umma_f16(d0 + 192, a1, b2, 1u);
+                            umma_f16(d0, a0, b0, kIdesc, on);
+                            umma_f16(d0 + 64, a0, b1, kIdesc, on);
+                            umma_f16(d0 + 64, a1, b0, kIdesc, 1u);
+                            umma_f16(d0 + 128, a0, b2, kIdesc, on);
+                            umma_f16(d0 + 128, a1, b1, kIdesc, 1u);
+                            umma_f16(d0 + 192, a0, b3, kIdesc, on);
+                            umma_f16(d0 + 192, a1, b2, kIdesc, 1u);
                         }
                         umma_commit(&sh.dig_empty[dg]);
                     }
@@ -410,7 +342,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
                                 : nullptr;
             for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl, ++tcount) {
                 const uint32_t acc = tcount % kAccStages;
-                if (!(ok = warp_wait(sh, &sh.acc_full[acc], (tcount / kAccStages) & 1u, a.err, lane))) break;
+                if (!(ok = tc_warp_wait(&sh.abort, &sh.acc_full[acc], (tcount / kAccStages) & 1u, a.err, lane))) break;
                 tc_fence_after();
                 const uint32_t c0 = sl * kN;
                 const uint32_t valid = min(kN, a.row_words - c0);
@@ -462,7 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
                     }
                     if (full) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 16; j += 4) sts_v4(srow + cc * 16 + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+                        for (uint32_t j = 0; j < 16; j += 4) sts_v4(smem_addr(srow + cc * 16 + j), v[j], v[j + 1], v[j + 2], v[j + 3]);
                     } else if (has) {
                         uint32_t *g = reinterpret_cast<uint32_t *>(orow) + c0 + cc * 16;
 #pragma unroll
@@ -498,8 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == kMmaWarp)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
