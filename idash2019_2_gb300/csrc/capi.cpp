@@ -142,7 +142,7 @@ idash_status upload_plan(idash_model *m, const Candidate &c, BuiltPlan &&b) {
     if ((s = upload(ctx, &m->d_terms, plan.terms)) != IDASH_OK) return s;
     if (c.kind == KernelKind::kTc) {
         if ((s = upload(ctx, &m->d_tc_a, plan.tc_a)) != IDASH_OK) return s;
-        if ((s = upload(ctx, &m->d_tc_bias, plan.tc_bias)) != IDASH_OK) return s;
+        if ((s = upload(ctx, &m->d_tc_out, plan.tc_out)) != IDASH_OK) return s;
     }
     if (m->form == Form::kTrlwe) {
         if ((s = upload(ctx, &m->d_var_ptr, plan.var_ptr)) != IDASH_OK) return s;
@@ -217,12 +217,13 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
         // CTA so the persistent grid balances; the block's coefficient digits
         // are loaded once per unit
         a.tc_a = m->d_tc_a;
-        a.tc_bias = m->d_tc_bias;
+        a.tc_out = m->d_tc_out;
         a.tc_a_max_bytes = uint32_t(tc_a_bytes(m->max_terms));
         const uint64_t tiles = uint64_t(a.n_blocks) * a.n_slices;
         const uint64_t want = std::max<uint64_t>(1, uint64_t(m->ctas) * 32);
         a.unit_slices = uint32_t(std::min<uint64_t>(a.n_slices, std::max<uint64_t>(1, (tiles + want - 1) / want)));
         a.units_per_block = (a.n_slices + a.unit_slices - 1) / a.unit_slices;
+        a.unit_slices = (a.n_slices + a.units_per_block - 1) / a.units_per_block;  // evenly
         a.n_units = a.n_blocks * a.units_per_block;
     }
     return a;
@@ -367,7 +368,7 @@ std::vector<Candidate> candidates(idash_model *m) {
     // with NUM_REGIONS = 1, and the LWE form), 64-column slices, K up to 192
     if ((ctx->opt_kernel == 0 || ctx->opt_kernel == 5) && (ctx->opt_slice_words == 0 || ctx->opt_slice_words == 64) &&
         (m->form == Form::kLwe || (m->form == Form::kTrlwe && m->tp.num_regions == 1))) {
-        Candidate c{KernelKind::kTc, kTcSliceWords, 1, 192, 0, 0, 1};
+        Candidate c{KernelKind::kTc, kTcSliceWords, 1, kTcMaxK, 0, 0, 1};
         out.push_back(c);
     }
     if (ctx->opt_kernel == 5) return out;
@@ -510,9 +511,9 @@ void idash_model::free_device() {
     cudaFree(d_out_index);
     cudaFree(d_out_row);
     cudaFree(d_tc_a);
-    cudaFree(d_tc_bias);
+    cudaFree(d_tc_out);
     d_tc_a = nullptr;
-    d_tc_bias = nullptr;
+    d_tc_out = nullptr;
     d_out_row = nullptr;
     d_blocks = nullptr;
     d_slots = nullptr;

@@ -127,7 +127,7 @@ struct idash_model {
     uint32_t *d_out_index = nullptr;
     uint32_t *d_out_row = nullptr;
     uint8_t *d_tc_a = nullptr;      // tensor-core plans: coefficient digits per block
-    uint32_t *d_tc_bias = nullptr;  // tensor-core plans: bias per output
+    idash::TcOut *d_tc_out = nullptr;  // tensor-core plans: constants per output
 
     // cached CUDA graph of the last device-path call
     cudaGraphExec_t graph = nullptr;

@@ -25,8 +25,7 @@
 //              registers), split them into digits, store them as the MMA's A
 //              (k-groups 16 bytes off a multiple of 128 apart, so that the
 //              eight groups of a row, one per lane, are in different banks);
-//   warp 8     lane 0 issues the MMAs: t0 over chunk g and t1 over chunk
-//              g - kLag, so that one tile's epilogue runs under the other's
+//   warp 8     issues the MMAs: t0 over chunk g and t1 over chunk g - kLag, so that one tile's epilogue runs under the other's
 //              MMAs although the two accumulators (2 x 256 columns) fill TMEM;
 //   warps 0-3  epilogue of t0, warps 4-7 of t1: each lane turns its digit sums
 //              into shifted words, three lanes exchange them (two shuffles per
@@ -253,69 +252,64 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
         }
     } else if (warp == kMmaWarp) {
         // ----------------------------------------------------------------- MMA
-        if (lane == 0) {
-            const uint32_t a_base = smem_addr(stages), t_base = smem_addr(table);
-            // where a tile is in the CTA's stream of chunks, and its columns
-            struct Cursor {
-                uint64_t i;  // item number
-                uint32_t c, s, round;
-                uint32_t w, idesc;
-                uint64_t b;  // descriptor of the tile's next K-step
-            } at[2] = {};
-            const uint64_t a_desc = umma_desc(a_base, kGroupBytes, 128);
-            // tile t over its next chunk; false: a wait ended
-            auto chunk = [&](uint32_t t, Cursor &x) {
-                if (x.c == 0) {
-                    uint32_t n0;
-                    tile_of(blockIdx.x + x.i * gridDim.x, t, n0, x.w);
-                    x.idesc = umma_idesc_f16(128, x.w);
-                    x.b = umma_desc(t_base + n0 * 16, 128, 128);
-                    if (x.i > 0) {
-                        if (!tc_wait(&sh.abort, &sh.acc_empty[t], uint32_t(x.i - 1) & 1u, a.err)) return false;
-                        tc_fence_after();
-                    }
+        const bool leader = elect_one();
+        // where a tile is in the CTA's stream of chunks, and its columns
+        struct Cursor {
+            uint64_t i;  // item number
+            uint32_t c, s, round;
+            uint32_t w, idesc;
+            uint64_t b;  // descriptor of the tile's next K-step
+        } at[2] = {};
+        const uint64_t a_desc = umma_desc(smem_addr(stages), kGroupBytes, 128);
+        const uint32_t t_base = smem_addr(table);
+        // tile t over its next chunk; false: a wait ended
+        auto chunk = [&](uint32_t t, Cursor &x) {
+            if (x.c == 0) {
+                uint32_t n0;
+                tile_of(blockIdx.x + x.i * gridDim.x, t, n0, x.w);
+                x.idesc = umma_idesc_f16(128, x.w);
+                x.b = umma_desc(t_base + n0 * 16, 128, 128);
+                if (x.i > 0) {
+                    if (!tc_wait(&sh.abort, &sh.acc_empty[t], uint32_t(x.i - 1) & 1u, a.err)) return false;
+                    tc_fence_after();
                 }
+            }
+            const uint64_t da = a_desc + x.s * (kStageBytes / 16);
+            if (leader) {
                 if (x.w) {
-                    const uint64_t da = a_desc + x.s * (kStageBytes / 16);
 #pragma unroll
                     for (uint32_t j = 0; j < kChunkWords / 16; ++j)
                         umma_f16(tmem + t * kTileMax, da + j * (2 * kGroupBytes / 16), x.b + j * 16, x.idesc,
                                  x.c + j > 0 ? 1u : 0u);
-                    x.b += (kChunkWords / 8) * (128 / 16);
                 }
-                if (++x.c == n_chunks) {
-                    umma_commit(&sh.acc_full[t]);
-                    x.c = 0;
-                    ++x.i;
-                }
-                return true;
-            };
-            auto next_stage = [](Cursor &x) {
-                if (++x.s == kStages) {
-                    x.s = 0;
-                    ++x.round;
-                }
-            };
-            bool ok = true;
-            for (uint32_t lead = 0; ok && at[1].i < my_items; ++lead) {
-                if (at[0].i < my_items) {
-                    ok = tc_wait(&sh.abort, &sh.a_full[at[0].s], at[0].round & 1u, a.err);
-                    if (!ok) break;
-                    tc_fence_after();
-                    ok = chunk(0, at[0]);
-                    next_stage(at[0]);
-                }
-                if (ok && lead >= kLag) {
-                    ok = chunk(1, at[1]);
-                    if (ok) umma_commit(&sh.a_empty[at[1].s]);
-                    next_stage(at[1]);
-                    lead = kLag;  // the counter only tells whether t1 has started
-                }
+                if (t == 1) umma_commit(&sh.a_empty[x.s]);
+                if (x.c + 1 == n_chunks) umma_commit(&sh.acc_full[t]);
             }
-            // every MMA issued has completed before TMEM is released
-            umma_commit(&sh.drain);
-            mbar_wait_bounded(&sh.drain, 0, nullptr);
+            __syncwarp();
+            x.b += (kChunkWords / 8) * (128 / 16);
+            if (++x.c == n_chunks) {
+                x.c = 0;
+                ++x.i;
+            }
+            if (++x.s == kStages) {
+                x.s = 0;
+                ++x.round;
+            }
+            return true;
+        };
+        bool ok = true;
+        for (uint32_t lead = 0; ok && at[1].i < my_items; lead = min(lead + 1, kLag)) {
+            if (at[0].i < my_items) {
+                ok = tc_wait(&sh.abort, &sh.a_full[at[0].s], at[0].round & 1u, a.err);
+                if (!ok) break;
+                tc_fence_after();
+                ok = chunk(0, at[0]);
+            }
+            if (ok && lead >= kLag) ok = chunk(1, at[1]);
         }
+        // every MMA issued has completed before TMEM is released
+        if (leader) umma_commit(&sh.drain);
+        mbar_wait_bounded(&sh.drain, 0, nullptr);
         __syncwarp();
     } else {
         // ------------------------------------------------------------ epilogue

@@ -333,7 +333,21 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
     k_max = std::min(k_max, lim.max_k / 16 * 16);
     if (k_max < 16) return "no K satisfies the exactness bound";
 
-    plan->tc_bias.assign(nm.bias.begin(), nm.bias.end());
+    plan->tc_out.resize(n_out);
+    for (uint64_t o = 0; o < n_out; ++o) {
+        int64_t s0 = 0, s1 = 0;  // K's bound keeps 128 times each below 2^22
+        for (uint64_t t = nm.nptr[o]; t < nm.nptr[o + 1]; ++t) {
+            const uint32_t c = nm.ncoef[t];
+            const int32_t c0 = int32_t((c + 128u) & 255u) - 128;
+            s0 += c0;
+            s1 += c0 + (int64_t(int32_t(c)) - c0) / 256;
+        }
+        TcOut &x = plan->tc_out[o];
+        x.bias = nm.bias[o];
+        x.offset = 128u * uint32_t(s0) + 0x01010100u * 128u * uint32_t(s1);
+        x.m0 = 0.75f - float(128 * s0) * 0x1p-24f;
+        x.m1 = 0.75f - float(128 * s1) * 0x1p-24f;
+    }
     plan->phase_begin.push_back(0);
     std::vector<uint64_t> win, merged;
     for (uint64_t o = 0; o < n_out;) {

@@ -80,6 +80,14 @@ struct PlanLimits {
     bool split = false;
 };
 
+// Tensor-core plans: one output's epilogue constants (score_tc.cu).
+struct TcOut {
+    uint32_t bias;
+    uint32_t offset;  // sum_s 256^s 128 S_s, S_0 = sum c0 and S_s = sum (c0 + c1) for s >= 1
+    float m0, m1;     // 0.75 - 128 S_0 2^-24 and 0.75 - 128 S_1 2^-24
+};
+static_assert(sizeof(TcOut) == 16, "one 16-byte load");
+
 struct Plan {
     std::vector<PlanBlock> blocks;
     // Blocks of phase p are [phase_begin[p], phase_begin[p + 1]), each phase
@@ -101,9 +109,9 @@ struct Plan {
     std::vector<uint32_t> block_max_row;  // per block: largest input row read
     std::vector<uint32_t> block_min_row;  // per block: smallest input row read (0 if none)
     // Tensor-core plans only (build_tc_plan): per block, the coefficient
-    // digits in the MMA's shared-memory layout, and every output's bias.
+    // digits in the MMA's shared-memory layout, and every output's constants.
     std::vector<uint8_t> tc_a;
-    std::vector<uint32_t> tc_bias;
+    std::vector<TcOut> tc_out;
 };
 
 // Tensor-core plans (build_tc_plan).  A block is up to kTcRows consecutive
@@ -116,19 +124,21 @@ struct Plan {
 // one 2D tensor copy), n_terms the block's nonzero terms, out_lo/out_hi its
 // outputs.
 //
-// Exactness (fp16 digits, fp32 accumulation): a ciphertext word x is split
-// into four balanced base-256 digits (x + 0x80808080 byte by byte, minus 128),
-// a coefficient c into c0 in [-128, 127] and c1 = (c - c0) / 256; product
-// digit sums for shift 8s are sums over K of at most two digit products, so
-// |sum| <= K * 128 * (128 + max|c1|).  The planner keeps that below 2^22
-// (where x + 1.5 * 2^23 is exact in fp32) by bounding K, and refuses models
-// with a coefficient outside two digits.
+// Exactness (fp16 digits, fp32 accumulation): a ciphertext word is split into
+// its four bytes b, a coefficient c into c0 in [-128, 127] and c1 = (c - c0) /
+// 256; digit sums for shift 8s are sums over K of at most two digit products,
+// so with balanced digits b - 128 |sum| <= K * 128 * (128 + max|c1|).  The
+// planner keeps that below 2^22 by bounding K: the accumulated sums of b
+// themselves then stay below 2^23, exact in fp32, and the balanced sum plus
+// 0.75 * 2^24 stays in one binade (score_tc.cu).  It refuses models with a
+// coefficient outside two digits.
 constexpr uint32_t kTcRows = 128;
+constexpr uint32_t kTcMaxK = 192;  // shared-memory bound on the padded K
 struct TcLimits {
-    uint32_t max_k = 192;  // shared-memory bound on the padded K
+    uint32_t max_k = kTcMaxK;
 };
 // Bytes of one block's coefficient digits: 2 digit planes x 128 rows x k_pad fp16.
-inline uint64_t tc_a_bytes(uint32_t k_pad) { return uint64_t(4) * kTcRows * k_pad; }
+constexpr uint64_t tc_a_bytes(uint32_t k_pad) { return uint64_t(4) * kTcRows * k_pad; }
 std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, bool *index_error);
 
 // Returns "" on success, else a message; *index_error is set when a term

@@ -63,15 +63,17 @@ struct ScoreArgs {
     uint64_t digest_base;         // a multiple of 4
     // KernelKind::kTc only.  tc_a: per block, the coefficient digits in the
     // MMA's shared-memory layout (PlanBlock::group_begin is the block's
-    // offset in 16-byte units, PlanBlock::n_groups its padded K); tc_bias:
-    // every output's bias.  Work unit u covers column slices
+    // offset in 16-byte units, PlanBlock::n_groups its padded K); tc_out:
+    // every output's constants.  Work unit u covers column slices
     // [(u % units_per_block) * unit_slices, + unit_slices) of block
     // block_lo + u / units_per_block.
     const uint8_t *tc_a;
-    const uint32_t *tc_bias;
+    const TcOut *tc_out;
     uint32_t unit_slices, units_per_block, n_units;
     uint32_t tc_a_max_bytes;      // shared-memory room for one block's digits
-    uint32_t tc_use_map;          // set by the launch: consecutive-row chunks come by 2D tensor copy
+    uint32_t unit_step_blocks, unit_step_parts;  // set by the launch: gridDim.x units in blocks and units of a block
+    uint32_t tc_use_map, tc_store_map;  // set by the launch: rows come, and outputs go, by tensor copies
+    uint32_t tc_a_stages, tc_dig_stages, tc_raw_stages;  // set by the launch: buffers of each kind
     // Multi-job launches (KernelKind::kWs only): n_jobs > 0 replaces the
     // per-launch input, output, row window, columns, bias rows and digest by
     // the job of each tile; jobs sorted by tile_begin, n_tiles their total.

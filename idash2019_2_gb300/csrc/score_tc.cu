@@ -9,41 +9,50 @@
 // digit products, as in the published tensor-core methods that emulate exact
 // or high-precision matrix products by splitting (Mukunoki, Ozaki, Ogita and
 // Imamura, "DGEMM using Tensor Cores, and Its Accurate and Reproducible
-// Versions", ISC 2020).  A ciphertext word x is written as four balanced
-// base-256 digits x = sum_i b_i 256^i (mod 2^32), b_i = byte_i(x + 0x80808080)
-// - 128 in [-128, 127]; a coefficient c as c0 + 256 c1, c0 in [-128, 127].
-// Digit products land in four accumulators by shift: D_s = sum over i + j = s
-// of A_j * B_i, s = 0..3 (seven MMAs per K-step), and
-//   out = sum_s 256^s D_s  (mod 2^32).
-// The planner bounds K so that every partial sum stays below 2^22 in
-// magnitude (plan.hpp), where fp32 holds integers exactly; the epilogue turns
-// D_s into an integer by adding 1.5 * 2^23 and reading the bits.
+// Versions", ISC 2020).  A ciphertext word is its four bytes x = sum_i b_i
+// 256^i; the fp16 bit pattern of a byte (a subnormal) is the value b * 2^-24,
+// so a byte is its own encoding.  A coefficient is c0 + 256 c1, c0 in [-128,
+// 127].  Digit products land in four accumulators by shift: D_s = sum over
+// i + j = s of A_j * B_i, s = 0..3, and out = sum_s 256^s D_s (mod 2^32).
+// The planner bounds K so that with balanced digits b - 128 every partial sum
+// stays below 2^22 units of 2^-24 (plan.hpp), so with b in [0, 255] below
+// 2^23, which fp32 holds exactly.  The epilogue adds 0.75 - 128 S_s 2^-24
+// (S_s: the output's digit sum that multiplies D_s): the result is 0.75 plus
+// the balanced sum, in [0.5, 1), where the last place is 2^-24 and the bits
+// are an integer; the plan's per-output constant puts 128 S_s back.
 //
-// Structure (one CTA of 10 warps per SM, persistent over work units of
-// (block, run of 64-column slices)):
-//   warp 4     producer: the block's coefficient digits (one bulk copy, kept
-//              in shared memory for the unit) and, per chunk of 32 rows, the
-//              rows' 64-column slices: one 2D tensor copy
-//              (cp.async.bulk.tensor) when the chunk's rows are consecutive,
-//              else one cp.async.bulk per row; completed on mbarriers;
-//   warps 6-9  converters: raw words -> four fp16 digit planes in the MMA's
-//              no-swizzle K-major layout;
-//   warp 5     allocates the 512 TMEM columns; lane 0 issues tcgen05.mma
-//              (M = 128, N = 64, K = 16) into a double-buffered set of four
-//              fp32 accumulators and commits to mbarriers;
-//   warps 0-3  epilogue: tcgen05.ld of the accumulators (warp w reads TMEM
-//              lanes 32w..32w+31, one output each), the digit recombination,
-//              bias and zeroed columns; each warp stages its 32 rows in
-//              shared memory and stores them row by row with coalesced
-//              16-byte streaming stores (no barrier across warps).
+// Structure (one CTA of 23 warps per SM, persistent over work units of
+// (block, run of 64-column slices)); each role's hand-offs take hundreds of
+// cycles, so the roles that would otherwise be bound by them come in teams
+// that take tiles or chunks in turn:
+//   warp 12     producer: per chunk of 32 rows, the rows' 64-column slices: one
+//               2D tensor copy when the chunk's rows are consecutive, else
+//               eight four-row gathers;
+//   warp 14     loads the block's coefficient digits (one bulk copy, kept in
+//               shared memory for the unit, the next unit's beside them where
+//               they fit);
+//   warps 15-22 converters, two teams of four for every other chunk: eight
+//               rows of a column -> one 16-byte row of each of the four byte
+//               planes, in the MMA's no-swizzle K-major layout with the
+//               planes side by side along N;
+//   warp 13     allocates the 512 TMEM columns and issues two tcgen05.mma
+//               per K = 16 step (M = 128: c0 times the four planes, N = 256,
+//               and c1 times the first three, N = 192, one accumulator to the
+//               right) into a double-buffered set of four fp32 accumulators;
+//   warps 0-11  epilogue, three teams of four for every third tile:
+//               tcgen05.ld of the accumulators (a warp reads 32 TMEM lanes,
+//               one output each), the digit recombination, bias and zeroed
+//               columns, staged in shared memory (128-byte swizzle) and
+//               stored by 2D tensor copies of 32 rows x 32 columns, or row by
+//               row where the 32 rows are not all wanted or not consecutive.
 // Every wait is bounded; a wait that expires records IDASH_ERR_DEVICE_TIMEOUT,
 // raises a CTA-wide abort flag that ends the other roles' waits, and each
 // role then waits (bounded) for its own copies and MMAs in flight before the
 // TMEM columns are freed.
 #include <cuda.h>
-#include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -58,32 +67,99 @@ namespace {
 constexpr uint32_t kN = kTcSliceWords;  // 64 columns per tile
 constexpr uint32_t kM = kTcRows;        // 128 outputs per block
 constexpr uint32_t kChunk = 32;         // rows per pipeline chunk (two MMA K-steps)
-constexpr uint32_t kRawStages = 4, kDigStages = 2, kAccStages = 2;
-constexpr uint32_t kRawRow = kN + 4;                    // words per row slice in a raw stage (bank padding)
-constexpr uint32_t kRawStageBytes = kChunk * kRawRow * 4;
-constexpr uint32_t kPlaneBytes = kChunk * kN * 2;       // one fp16 digit plane of a chunk
-constexpr uint32_t kDigStageBytes = 4 * kPlaneBytes;
-constexpr uint32_t kOutRow = kN + 4;                    // words per output row in the staging buffer
-constexpr uint32_t kOutBytes = kM * kOutRow * 4;
+constexpr uint32_t kMaxChunks = kTcMaxK / kChunk;
+constexpr uint32_t kAccStages = 2;
+constexpr uint32_t kMaxAStages = 2, kMaxRawStages = 8, kMaxDigStages = 4;
+constexpr uint32_t kRawStageBytes = kChunk * kN * 4;
+constexpr uint32_t kGroupBytes = 4 * kN * 16;           // 8 rows of the four planes
+constexpr uint32_t kDigStageBytes = (kChunk / 8) * kGroupBytes;
+constexpr uint32_t kOutBox = 32 * 32 * 4;               // one stored box: 32 rows x 32 columns
 constexpr uint32_t kHeader = 1024;
-constexpr uint32_t kThreads = 320;
-constexpr uint32_t kProducerWarp = 4, kMmaWarp = 5, kConvWarp0 = 6;
+// Warps: kEpi teams of eight (one, or one per accumulator stage), then one
+// each of producer, MMA and digit loads, then kConv converter teams of
+// kConvWarps.  A parity tells only two successive phases of a barrier apart,
+// so a team must meet all phases of the stages it waits for in turn: a stage
+// belongs to one team.
+constexpr uint32_t kEpiWarps = 8;
+constexpr uint32_t tc_threads(uint32_t epi, uint32_t conv, uint32_t conv_warps) {
+    return 32 * (kEpiWarps * epi + 3 + conv_warps * conv);
+}
 constexpr uint32_t kTmemCols = 512;                     // 2 stages x 4 accumulators x 64 columns
-constexpr uint32_t kIdesc = umma_idesc_f16(kM, kN);
-constexpr uint32_t kMagic = 0x4B400000u;                // bits of 1.5 * 2^23
+constexpr uint32_t kIdescAll = umma_idesc_f16(kM, 4 * kN), kIdescHigh = umma_idesc_f16(kM, 3 * kN);
+constexpr uint32_t kMagic = 0x3F400000u;                // bits of 0.75
 constexpr uint32_t kMagicSum = kMagic + (kMagic << 8) + (kMagic << 16) + (kMagic << 24);
 // one CTA per SM, so the CTA owns all of TMEM
 constexpr size_t kMinSmem = 120 * 1024;
+constexpr size_t kMaxSmem = 227 * 1024;
+
+// Teams and buffers for a plan whose largest padded K is k.  Small K: the
+// epilogue is most of the work (two teams, one per accumulator stage); large
+// K: the conversion is.  Then the first set of buffers that fits.  Raw and
+// digit stages are multiples of the converter teams (see above).
+struct TcShape {
+    uint32_t epi, conv, conv_warps;
+    uint32_t a_stages;    // blocks' coefficient digits
+    uint32_t dig_stages;  // chunks of byte planes
+    uint32_t raw_stages;  // chunks of ciphertext words
+    constexpr size_t smem(uint32_t k) const {
+        const size_t n = kHeader + a_stages * size_t(tc_a_bytes(k)) + dig_stages * size_t(kDigStageBytes) +
+                         raw_stages * size_t(kRawStageBytes) + kEpiWarps * epi * size_t(kOutBox);
+        return n < kMinSmem ? kMinSmem : n;
+    }
+};
+constexpr TcShape kTcShapes[] = {{2, 2, 2, 2, 4, 6}, {2, 2, 2, 2, 4, 4}, {2, 2, 2, 1, 4, 6}, {2, 2, 2, 1, 4, 4},
+                                 {1, 3, 4, 1, 3, 6}};
+const TcShape *tc_shape(uint32_t k) {
+    for (const TcShape &x : kTcShapes)
+        if (x.smem(k) <= kMaxSmem) return &x;
+    return nullptr;
+}
 
 struct TcBars {
-    uint64_t a_full, a_empty, drain;
-    uint64_t raw_full[kRawStages], raw_empty[kRawStages];
-    uint64_t dig_full[kDigStages], dig_empty[kDigStages];
+    uint64_t a_full[kMaxAStages], a_empty[kMaxAStages], drain;
+    uint64_t raw_full[kMaxRawStages], raw_empty[kMaxRawStages];
+    uint64_t dig_full[kMaxDigStages], dig_empty[kMaxDigStages];
     uint64_t acc_full[kAccStages], acc_empty[kAccStages];
     uint32_t tmem_base;
     uint32_t abort;
 };
 static_assert(sizeof(TcBars) <= kHeader, "barrier area");
+
+// A position in a ring of n stages; parity of the round.
+struct Ring {
+    uint32_t s = 0, round = 0;
+    __device__ __forceinline__ void next(uint32_t n) {
+        if (++s == n) {
+            s = 0;
+            ++round;
+        }
+    }
+};
+
+// A 16-byte shared load that stays before the barrier that follows it.
+__device__ __forceinline__ uint4 lds_v4_ordered(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.volatile.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// x + m and y + m as floats, each rounded to nearest, in one instruction.
+__device__ __forceinline__ void add2(uint32_t &x, uint32_t &y, float m) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\t"
+        "add.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+r"(x), "+r"(y)
+        : "f"(m));
+}
 
 __device__ __forceinline__ void expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
@@ -100,331 +176,511 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-__device__ __forceinline__ uint4 lds_v4p(const uint32_t *p) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr(p)));
-    return v;
+// Four rows' boxes (one row high) at column x, one after another in shared memory.
+__device__ __forceinline__ void tma_gather4(void *dst, const CUtensorMap *map, int32_t x, const int32_t (&y)[4],
+                                            uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+        "%3, %4, %5, %6}], [%7];" ::"r"(smem_addr(dst)),
+        "l"(map), "r"(x), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(smem_addr(bar))
+        : "memory");
 }
 
-// fp16x2 bits {lo: v_lo - 128, hi: v_hi - 128} from r = [v_lo, 0x64, v_hi, 0x64]
-// (fp16 1024 + v, exact) minus 1152.
-__device__ __forceinline__ uint32_t digits_minus_128(uint32_t r) {
-    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&r), __half2(__half(1152.f), __half(1152.f)));
-    return *reinterpret_cast<const uint32_t *>(&h);
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int32_t x, int32_t y, uint32_t src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x),
+                 "r"(y), "r"(src)
+                 : "memory");
 }
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// At most kLeft of this thread's store groups still read shared memory.
+template <int kLeft>
+__device__ __forceinline__ void bulk_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kLeft) : "memory");
+}
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-struct Unit {
-    PlanBlock blk;
-    uint32_t s0, s1, k_pad, n_chunks;
+// The CTA's work units blockIdx.x, + gridDim.x, ...: unit u is slices [s0, s1)
+// of block `block`.  Stepped without a division.
+struct Units {
+    uint32_t u, block, part;
+    __device__ __forceinline__ explicit Units(const ScoreArgs &a)
+        : u(blockIdx.x), block(blockIdx.x / a.units_per_block), part(blockIdx.x % a.units_per_block) {}
+    __device__ __forceinline__ bool valid(const ScoreArgs &a) const { return u < a.n_units; }
+    __device__ __forceinline__ void next(const ScoreArgs &a) {
+        u += gridDim.x;
+        block += a.unit_step_blocks;
+        part += a.unit_step_parts;
+        if (part >= a.units_per_block) {
+            part -= a.units_per_block;
+            ++block;
+        }
+    }
+    __device__ __forceinline__ uint32_t s0(const ScoreArgs &a) const { return part * a.unit_slices; }
+    __device__ __forceinline__ uint32_t s1(const ScoreArgs &a) const {
+        return min((part + 1) * a.unit_slices, a.n_slices);
+    }
+    __device__ __forceinline__ const PlanBlock *header(const ScoreArgs &a) const {
+        return a.blocks + a.block_lo + block;
+    }
 };
 
-__device__ __forceinline__ Unit unit_of(const ScoreArgs &a, uint32_t u) {
-    Unit x;
-    x.blk = a.blocks[a.block_lo + u / a.units_per_block];
-    x.s0 = (u % a.units_per_block) * a.unit_slices;
-    x.s1 = min(x.s0 + a.unit_slices, a.n_slices);
-    x.k_pad = x.blk.n_groups;
-    x.n_chunks = (x.k_pad + kChunk - 1) / kChunk;
-    return x;
+// Padded K of the CTA's units, each read one unit ahead of its use.
+struct UnitDepths {
+    Units ahead;
+    uint32_t pending;
+    __device__ __forceinline__ explicit UnitDepths(const ScoreArgs &a) : ahead(a), pending(0) { fetch(a); }
+    __device__ __forceinline__ void fetch(const ScoreArgs &a) {
+        if (ahead.valid(a)) pending = ahead.header(a)->n_groups;
+    }
+    __device__ __forceinline__ uint32_t next(const ScoreArgs &a) {
+        const uint32_t k = pending;
+        ahead.next(a);
+        fetch(a);
+        return k;
+    }
+};
+
+// Bit i: column c0 + i is in [lo, hi), i < 32.
+__device__ __forceinline__ uint32_t columns_in(uint32_t c0, uint32_t lo, uint32_t hi) {
+    const uint32_t from = lo > c0 ? min(lo - c0, 32u) : 0u, to = hi > c0 ? min(hi - c0, 32u) : 0u;
+    return from < to ? (0xFFFFFFFFu >> (32u - (to - from))) << from : 0u;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_score_tc(const ScoreArgs a, const __grid_constant__ CUtensorMap rows_map) {
+// The launch's tensor maps: rows (boxes of 64 columns x 32 rows), row
+// gathers (64 x 1) and outputs (32 x 32, 128-byte swizzle).
+struct TcMaps {
+    CUtensorMap rows, gather, out;
+};
+
+// n (at most 32) rows that one box does not hold, slots slot .. slot + n - 1,
+// into a raw stage: four-row gathers, or one copy per row where the launch has
+// no tensor maps.  The whole warp calls it.
+__device__ __noinline__ void load_rows(const ScoreArgs &a, const CUtensorMap &gather, uint32_t slot, uint32_t n,
+                                       uint32_t c0, uint8_t *dst, uint64_t *full, uint32_t lane) {
+    // the row of slot i (the last ones repeated), 0 for one outside the input
+    auto row_of = [&](uint32_t i) {
+        const uint32_t r = a.slots[slot + min(i, n - 1)].row - a.row_base;
+        if (r < a.n_rows) return r;
+        report_error(a.err, kDevBadIndex);
+        return 0u;
+    };
+    fence_proxy_async_smem();  // after the converters' reads of the stage
+    if (n && a.n_rows) {
+        if (a.tc_use_map) {
+            if (4 * lane < n) {
+                const int32_t y[4] = {int32_t(row_of(4 * lane)), int32_t(row_of(4 * lane + 1)),
+                                      int32_t(row_of(4 * lane + 2)), int32_t(row_of(4 * lane + 3))};
+                expect_tx(full, 4 * kN * 4);
+                tma_gather4(dst + lane * (4 * kN * 4), &gather, int32_t(c0), y, full);
+            }
+        } else if (lane < n) {
+            const uint32_t bytes = ((min(kN, a.row_words - c0) + 3u) & ~3u) * 4u;
+            const uint32_t r = row_of(lane);
+            expect_tx(full, bytes);
+            bulk_g2s(dst + lane * (kN * 4), a.in + uint64_t(r) * a.in_stride + uint64_t(c0) * 4, bytes, full);
+        }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(full);
+}
+
+template <uint32_t kEpi, uint32_t kConv, uint32_t kConvWarps>
+__global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps), 1)
+    k_score_tc(const __grid_constant__ ScoreArgs a, const __grid_constant__ TcMaps maps) {
+    constexpr uint32_t kProducerWarp = kEpiWarps * kEpi, kMmaWarp = kProducerWarp + 1, kDigitWarp = kMmaWarp + 1;
+    constexpr uint32_t kConvWarp0 = kDigitWarp + 1;
     extern __shared__ __align__(1024) uint8_t smem[];
     TcBars &sh = *reinterpret_cast<TcBars *>(smem);
-    uint8_t *smA = smem + kHeader;
-    uint8_t *raw = smA + a.tc_a_max_bytes;
-    uint8_t *dig = raw + kRawStages * kRawStageBytes;
-    uint8_t *stage_out = dig + kDigStages * kDigStageBytes;
+    uint8_t *stage_out = smem + kHeader;
+    uint8_t *smA = stage_out + kEpiWarps * kEpi * kOutBox;
+    uint8_t *dig = smA + a.tc_a_stages * a.tc_a_max_bytes;
+    uint8_t *raw = dig + a.tc_dig_stages * kDigStageBytes;
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 
     if (threadIdx.x == 0) {
-        mbar_init(&sh.a_full, 1);
-        mbar_init(&sh.a_empty, 1);
-        mbar_init(&sh.drain, 1);
-        for (uint32_t s = 0; s < kRawStages; ++s) {
-            mbar_init(&sh.raw_full[s], 1);
-            mbar_init(&sh.raw_empty[s], 4);
+        for (uint32_t s = 0; s < kMaxAStages; ++s) {
+            mbar_init(&sh.a_full[s], 1);
+            mbar_init(&sh.a_empty[s], 1);
         }
-        for (uint32_t s = 0; s < kDigStages; ++s) {
-            mbar_init(&sh.dig_full[s], 4);
+        mbar_init(&sh.drain, 1);
+        for (uint32_t s = 0; s < kMaxRawStages; ++s) {
+            mbar_init(&sh.raw_full[s], 1);
+            mbar_init(&sh.raw_empty[s], kConvWarps);
+        }
+        for (uint32_t s = 0; s < kMaxDigStages; ++s) {
+            mbar_init(&sh.dig_full[s], kConvWarps);
             mbar_init(&sh.dig_empty[s], 1);
         }
         for (uint32_t s = 0; s < kAccStages; ++s) {
             mbar_init(&sh.acc_full[s], 1);
-            mbar_init(&sh.acc_empty[s], 4);
+            mbar_init(&sh.acc_empty[s], kEpiWarps);
         }
         sh.abort = 0;
         fence_mbar_init();
     }
-    if (warp == kMmaWarp) {
-        tmem_alloc(&sh.tmem_base, kTmemCols);
-    }
+    if (warp == kMmaWarp) tmem_alloc(&sh.tmem_base, kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh.tmem_base;
 
-    if (warp == kProducerWarp) {
-        // ------------------------------------------------------------ producer
-        uint32_t rc = 0, a_loads = 0;
-        bool ok = true;
-        for (uint32_t u = blockIdx.x, uc = 0; ok && u < a.n_units; u += gridDim.x, ++uc) {
-            const Unit x = unit_of(a, u);
-            if (uc > 0 && !(ok = tc_warp_wait(&sh.abort, &sh.a_empty, (uc - 1) & 1u, a.err, lane))) break;
-            if (lane == 0) {
-                const uint32_t bytes = 4u * kM * x.k_pad;  // tc_a_bytes(k_pad): two fp16 digit planes
-                fence_proxy_async_smem();
-                mbar_arrive_expect_tx(&sh.a_full, bytes);
-                bulk_g2s(smA, a.tc_a + uint64_t(x.blk.group_begin) * 16, bytes, &sh.a_full);
+    if (warp == kDigitWarp) {
+        // -------------------------------------------- coefficient digit loads
+        if (lane == 0) {
+            Ring ra;
+            uint32_t loads = 0;
+            for (Units w(a); w.valid(a); w.next(a)) {
+                const PlanBlock *h = w.header(a);
+                const uint32_t bytes = uint32_t(tc_a_bytes(h->n_groups));
+                const uint8_t *src = a.tc_a + uint64_t(h->group_begin) * 16;
+                if (ra.round > 0 && !tc_wait(&sh.abort, &sh.a_empty[ra.s], (ra.round - 1) & 1u, a.err)) break;
+                mbar_arrive_expect_tx(&sh.a_full[ra.s], bytes);
+                bulk_g2s(smA + ra.s * a.tc_a_max_bytes, src, bytes, &sh.a_full[ra.s]);
+                ++loads;
+                ra.next(a.tc_a_stages);
             }
-            ++a_loads;
-            for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl) {
+            // let every copy land: the last fill of each buffer (immediate when nothing aborted)
+            for (uint32_t k = 1; k <= a.tc_a_stages && k <= loads; ++k) {
+                const uint32_t j = loads - k;
+                mbar_wait_bounded(&sh.a_full[j % a.tc_a_stages], (j / a.tc_a_stages) & 1u, nullptr);
+            }
+        }
+        __syncwarp();
+    } else if (warp == kProducerWarp) {
+        // ------------------------------------------------------------ producer
+        // The block header is read two units ahead and the rows one unit
+        // ahead, so that the loop below issues copies and nothing else: with
+        // the lookups in it, it took 850 cycles per chunk and bound the kernel.
+        struct Rows {
+            uint32_t n_slots, slot_begin, runs, n_chunks;  // runs: the block's consecutive-chunk mask
+            uint32_t first;                                // lane c: first row of chunk c
+        };
+        const bool leader = elect_one();
+        Units head(a);
+        PlanBlock blk{};
+        Rows next{};
+        auto fetch_header = [&]() {
+            if (head.valid(a)) blk = *head.header(a);
+            head.next(a);
+        };
+        auto fetch_rows = [&]() {  // of the block header last read
+            next = Rows{blk.n_slots, blk.slot_begin, blk.term_begin, (blk.n_groups + kChunk - 1) / kChunk, 0};
+            if (kChunk * lane < next.n_slots) next.first = a.slots[next.slot_begin + kChunk * lane].row - a.row_base;
+        };
+        fetch_header();
+        fetch_rows();
+        fetch_header();
+        Ring rr;
+        uint32_t rc = 0;
+        bool ok = true;
+        for (Units w(a); ok && w.valid(a); w.next(a)) {
+            const Rows x = next;
+            fetch_rows();
+            fetch_header();
+            // chunks that one tensor copy loads: consecutive rows, all inside the input
+            const uint32_t here = kChunk * lane < x.n_slots ? min(kChunk, x.n_slots - kChunk * lane) : 0u;
+            const uint32_t boxes = __ballot_sync(0xFFFFFFFFu, here && a.tc_use_map && ((x.runs >> lane) & 1u) &&
+                                                                  x.first < a.n_rows && here <= a.n_rows - x.first);
+            uint32_t r0[kMaxChunks];
+#pragma unroll
+            for (uint32_t c = 0; c < kMaxChunks; ++c) r0[c] = __shfl_sync(0xFFFFFFFFu, x.first, c);
+            const uint32_t s1 = w.s1(a);
+            for (uint32_t sl = w.s0(a); ok && sl < s1; ++sl) {
                 const uint32_t c0 = sl * kN;
-                const uint32_t valid = min(kN, a.row_words - c0);
-                const uint32_t copy_bytes = ((valid + 3u) & ~3u) * 4u;
-                for (uint32_t c = 0; c < x.n_chunks; ++c) {
-                    const uint32_t st = rc % kRawStages;
-                    if (rc >= kRawStages &&
-                        !(ok = tc_warp_wait(&sh.abort, &sh.raw_empty[st], ((rc / kRawStages) - 1) & 1u, a.err, lane)))
+#pragma unroll
+                for (uint32_t c = 0; c < kMaxChunks; ++c) {
+                    if (c >= x.n_chunks) break;
+                    uint64_t *full = &sh.raw_full[rr.s];
+                    uint8_t *dst = raw + rr.s * kRawStageBytes;
+                    if (rr.round > 0 && !(ok = tc_wait(&sh.abort, &sh.raw_empty[rr.s], (rr.round - 1) & 1u, a.err)))
                         break;
-                    if (lane == 0) fence_proxy_async_smem();
-                    __syncwarp();
-                    const uint32_t k_lo = c * kChunk, k_hi = min(k_lo + kChunk, uint32_t(x.blk.n_slots));
-                    uint8_t *dst = raw + st * kRawStageBytes;
-                    if (a.tc_use_map && k_hi > k_lo && ((x.blk.term_begin >> c) & 1u)) {
-                        // consecutive rows: the whole chunk (32 rows x 68 words) in one tensor copy
-                        if (lane == 0) {
-                            const uint32_t r0 = a.slots[x.blk.slot_begin + k_lo].row - a.row_base;
-                            if (r0 >= a.n_rows || r0 + (k_hi - k_lo) > a.n_rows) {
-                                report_error(a.err, kDevBadIndex);
-                            } else {
-                                expect_tx(&sh.raw_full[st], kRawStageBytes);
-                                tma_load_2d(dst, &rows_map, int32_t(c0), int32_t(r0), &sh.raw_full[st]);
-                            }
+                    if ((boxes >> c) & 1u) {
+                        if (leader) {
+                            fence_proxy_async_smem();  // after the converters' reads of the stage
+                            mbar_arrive_expect_tx(full, kRawStageBytes);
+                            tma_load_2d(dst, &maps.rows, int32_t(c0), int32_t(r0[c]), full);
                         }
                     } else {
-                        for (uint32_t k = k_lo + lane; k < k_hi; k += 32) {
-                            const uint32_t r = a.slots[x.blk.slot_begin + k].row - a.row_base;
-                            if (r >= a.n_rows) {
-                                report_error(a.err, kDevBadIndex);
-                                continue;
-                            }
-                            expect_tx(&sh.raw_full[st], copy_bytes);
-                            bulk_g2s(dst + (k - k_lo) * kRawRow * 4,
-                                     a.in + uint64_t(r) * a.in_stride + uint64_t(c0) * 4, copy_bytes,
-                                     &sh.raw_full[st]);
-                        }
+                        load_rows(a, maps.gather, x.slot_begin + kChunk * c,
+                                  x.n_slots > kChunk * c ? min(kChunk, x.n_slots - kChunk * c) : 0u, c0, dst, full,
+                                  lane);
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh.raw_full[st]);
                     ++rc;
+                    rr.next(a.tc_raw_stages);
                 }
             }
         }
         // let every copy this CTA issued land: the last fill of each raw
-        // stage and the last digit load (immediate when nothing aborted)
+        // stage (immediate when nothing aborted)
         if (lane == 0) {
-            for (uint32_t k = 1; k <= kRawStages && k <= rc; ++k) {
+            for (uint32_t k = 1; k <= a.tc_raw_stages && k <= rc; ++k) {
                 const uint32_t j = rc - k;
-                mbar_wait_bounded(&sh.raw_full[j % kRawStages], (j / kRawStages) & 1u, nullptr);
+                mbar_wait_bounded(&sh.raw_full[j % a.tc_raw_stages], (j / a.tc_raw_stages) & 1u, nullptr);
             }
-            if (a_loads) mbar_wait_bounded(&sh.a_full, (a_loads - 1) & 1u, nullptr);
         }
+        __syncwarp();
     } else if (warp >= kConvWarp0) {
         // ---------------------------------------------------------- converters
-        // thread -> row pair kp (rows 2kp, 2kp+1 of the chunk) and columns
-        // nl + 8i: raw reads and digit stores both hit 32 distinct banks
-        const uint32_t cw = warp - kConvWarp0;
-        const uint32_t kp = 4 * cw + lane / 8, nl = lane % 8;
-        uint32_t rc = 0;
+        // unit q of a chunk: rows 8 (q / 64) .. + 7 of column q % 64.  A warp's
+        // loads are 32 consecutive words, its stores 32 consecutive 16-byte rows.
+        constexpr uint32_t kTeamThreads = 32 * kConvWarps, kUnits = kN * (kChunk / 8) / kTeamThreads;
+        const uint32_t team = (warp - kConvWarp0) / kConvWarps;
+        const uint32_t tid = (warp - kConvWarp0) % kConvWarps * 32 + lane;
+        uint32_t turn = 0;
+        Ring rr, rd;
         bool ok = true;
-        for (uint32_t u = blockIdx.x; ok && u < a.n_units; u += gridDim.x) {
-            const Unit x = unit_of(a, u);
-            for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl) {
-                for (uint32_t c = 0; c < x.n_chunks; ++c, ++rc) {
-                    const uint32_t st = rc % kRawStages, dg = rc % kDigStages;
-                    if (!(ok = tc_warp_wait(&sh.abort, &sh.raw_full[st], (rc / kRawStages) & 1u, a.err, lane))) break;
-                    if (rc >= kDigStages &&
-                        !(ok = tc_warp_wait(&sh.abort, &sh.dig_empty[dg], ((rc / kDigStages) - 1) & 1u, a.err, lane)))
-                        break;
-                    const uint32_t rows = min(kChunk, x.k_pad - c * kChunk);
-                    if (2 * kp < rows) {
-                        const uint32_t *rw =
-                            reinterpret_cast<const uint32_t *>(raw + st * kRawStageBytes) + 2 * kp * kRawRow + nl;
-                        uint32_t *dp = reinterpret_cast<uint32_t *>(dig + dg * kDigStageBytes) + (kp / 4) * 256 +
-                                       nl * 4 + (kp % 4);
+        UnitDepths depths(a);
+        for (Units w(a); ok && w.valid(a); w.next(a)) {
+            const uint32_t k_pad = depths.next(a);
+            for (uint32_t n = w.s1(a) - w.s0(a); ok && n > 0; --n) {
+                for (uint32_t k0 = 0; k0 < k_pad; k0 += kChunk) {
+                    const bool mine = turn == team;
+                    if (++turn == kConv) turn = 0;
+                    if (!mine) {
+                        rr.next(a.tc_raw_stages);
+                        rd.next(a.tc_dig_stages);
+                        continue;
+                    }
+                    if (!(ok = tc_warp_wait(&sh.abort, &sh.raw_full[rr.s], rr.round & 1u, a.err, lane))) break;
+                    const uint32_t groups = min(kChunk, k_pad - k0) / 8;
+                    const uint32_t src = smem_addr(raw + rr.s * kRawStageBytes);
+                    const uint32_t dst = smem_addr(dig + rd.s * kDigStageBytes);
+                    // All of the raw stage's words first: it is free once they
+                    // are here.  Volatile loads: with plain ones the compiler
+                    // moved them below the arrival and the wait that follow.
+                    uint32_t w[kUnits][8];
 #pragma unroll
-                        for (uint32_t i = 0; i < kN / 8; ++i) {
-                            const uint32_t ya = rw[8 * i] + 0x80808080u, yb = rw[kRawRow + 8 * i] + 0x80808080u;
-                            const uint32_t lo = __byte_perm(ya, yb, 0x5140), hi = __byte_perm(ya, yb, 0x7362);
-                            constexpr uint32_t k64 = 0x64646464u;
-                            uint32_t *q = dp + 32 * i;
-                            q[0] = digits_minus_128(__byte_perm(lo, k64, 0x4140));
-                            q[kPlaneBytes / 4] = digits_minus_128(__byte_perm(lo, k64, 0x4342));
-                            q[2 * kPlaneBytes / 4] = digits_minus_128(__byte_perm(hi, k64, 0x4140));
-                            q[3 * kPlaneBytes / 4] = digits_minus_128(__byte_perm(hi, k64, 0x4342));
+                    for (uint32_t x = 0; x < kUnits; ++x) {
+                        const uint32_t q = x * kTeamThreads + tid, g = q / kN, col = q % kN;
+                        if (g >= groups) break;
+#pragma unroll
+                        for (uint32_t r = 0; r < 8; ++r)
+                            asm volatile("ld.volatile.shared.u32 %0, [%1];"
+                                         : "=r"(w[x][r])
+                                         : "r"(src + ((8 * g + r) * kN + col) * 4)
+                                         : "memory");
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.raw_empty[rr.s]);
+                    if (rd.round > 0 &&
+                        !(ok = tc_warp_wait(&sh.abort, &sh.dig_empty[rd.s], (rd.round - 1) & 1u, a.err, lane)))
+                        break;
+#pragma unroll
+                    for (uint32_t x = 0; x < kUnits; ++x) {
+                        const uint32_t q = x * kTeamThreads + tid, g = q / kN, col = q % kN;
+                        if (g >= groups) break;
+                        uint32_t p[4][4];
+#pragma unroll
+                        for (uint32_t r = 0; r < 4; ++r) {
+                            const uint32_t lo = __byte_perm(w[x][2 * r], w[x][2 * r + 1], 0x5140);
+                            const uint32_t hi = __byte_perm(w[x][2 * r], w[x][2 * r + 1], 0x7362);
+                            p[0][r] = __byte_perm(lo, 0u, 0x4140);
+                            p[1][r] = __byte_perm(lo, 0u, 0x4342);
+                            p[2][r] = __byte_perm(hi, 0u, 0x4140);
+                            p[3][r] = __byte_perm(hi, 0u, 0x4342);
                         }
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i)
+                            sts_v4(dst + g * kGroupBytes + (i * kN + col) * 16, p[i][0], p[i][1], p[i][2], p[i][3]);
                     }
                     fence_proxy_async_smem();  // the digits are read by the tensor cores (async proxy)
                     __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive(&sh.raw_empty[st]);
-                        mbar_arrive(&sh.dig_full[dg]);
-                    }
+                    if (lane == 0) mbar_arrive(&sh.dig_full[rd.s]);
+                    rr.next(a.tc_raw_stages);
+                    rd.next(a.tc_dig_stages);
                 }
             }
         }
     } else if (warp == kMmaWarp) {
         // ----------------------------------------------------------------- MMA
-        if (lane == 0) {
-            uint32_t rc = 0, tcount = 0;
-            bool ok = true;
-            const uint32_t a_base = smem_addr(smA), d_base = smem_addr(dig);
-            for (uint32_t u = blockIdx.x, uc = 0; ok && u < a.n_units; u += gridDim.x, ++uc) {
-                const Unit x = unit_of(a, u);
-                if (!(ok = tc_wait(&sh.abort, &sh.a_full, uc & 1u, a.err))) break;
-                const uint32_t a_plane = x.k_pad * 256;  // bytes per coefficient digit plane
-                for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl, ++tcount) {
-                    const uint32_t acc = tcount % kAccStages;
-                    if (tcount >= kAccStages &&
-                        !(ok = tc_wait(&sh.abort, &sh.acc_empty[acc], ((tcount / kAccStages) - 1) & 1u, a.err)))
-                        break;
+        Ring rd, ra, rt;
+        bool ok = true;
+        const bool leader = elect_one();
+        const uint64_t a_desc = umma_desc(smem_addr(smA), 2048, 128);
+        const uint64_t d_desc = umma_desc(smem_addr(dig), kGroupBytes, 128);
+        UnitDepths depths(a);
+        for (Units w(a); ok && w.valid(a); w.next(a)) {
+            const uint32_t k_pad = depths.next(a);
+            if (!(ok = tc_wait(&sh.abort, &sh.a_full[ra.s], ra.round & 1u, a.err))) break;
+            const uint64_t a_unit = a_desc + ra.s * (a.tc_a_max_bytes / 16);
+            const uint32_t plane = k_pad * 16;  // 16-byte units per coefficient digit plane
+            for (uint32_t n = w.s1(a) - w.s0(a); ok && n > 0; --n) {
+                if (rt.round > 0 && !(ok = tc_wait(&sh.abort, &sh.acc_empty[rt.s], (rt.round - 1) & 1u, a.err))) break;
+                tc_fence_after();
+                const uint32_t d0 = tmem + rt.s * (4 * kN);
+                uint64_t a0 = a_unit;
+                for (uint32_t k0 = 0; k0 < k_pad; k0 += kChunk) {
+                    if (!(ok = tc_wait(&sh.abort, &sh.dig_full[rd.s], rd.round & 1u, a.err))) break;
                     tc_fence_after();
-                    const uint32_t d0 = tmem + acc * 256;
-                    for (uint32_t c = 0; c < x.n_chunks; ++c, ++rc) {
-                        const uint32_t dg = rc % kDigStages;
-                        if (!(ok = tc_wait(&sh.abort, &sh.dig_full[dg], (rc / kDigStages) & 1u, a.err))) break;
-                        tc_fence_after();
-                        const uint32_t steps = min(kChunk, x.k_pad - c * kChunk) / 16;
-                        const uint32_t b_base = d_base + dg * kDigStageBytes;
-                        for (uint32_t j = 0; j < steps; ++j) {
-                            const uint32_t s = c * 2 + j, on = s > 0 ? 1u : 0u;
-                            const uint64_t a0 = umma_desc(a_base + s * 4096, 2048, 128);
-                            const uint64_t a1 = umma_desc(a_base + a_plane + s * 4096, 2048, 128);
-                            const uint64_t b0 = umma_desc(b_base + j * 2048, 1024, 128);
-                            const uint64_t b1 = umma_desc(b_base + kPlaneBytes + j * 2048, 1024, 128);
-                            const uint64_t b2 = umma_desc(b_base + 2 * kPlaneBytes + j * 2048, 1024, 128);
-                            const uint64_t b3 = umma_desc(b_base + 3 * kPlaneBytes + j * 2048, 1024, 128);
-                            umma_f16(d0, a0, b0, kIdesc, on);
-                            umma_f16(d0 + 64, a0, b1, kIdesc, on);
-                            umma_f16(d0 + 64, a1, b0, kIdesc, 1u);
-                            umma_f16(d0 + 128, a0, b2, kIdesc, on);
-                            umma_f16(d0 + 128, a1, b1, kIdesc, 1u);
-                            umma_f16(d0 + 192, a0, b3, kIdesc, on);
-                            umma_f16(d0 + 192, a1, b2, kIdesc, 1u);
+                    const uint64_t b0 = d_desc + rd.s * (kDigStageBytes / 16);
+                    if (leader) {
+                        umma_f16(d0, a0, b0, kIdescAll, k0 > 0 ? 1u : 0u);
+                        umma_f16(d0 + kN, a0 + plane, b0, kIdescHigh, 1u);
+                        if (k_pad - k0 > 16) {
+                            umma_f16(d0, a0 + 256, b0 + 2 * kGroupBytes / 16, kIdescAll, 1u);
+                            umma_f16(d0 + kN, a0 + plane + 256, b0 + 2 * kGroupBytes / 16, kIdescHigh, 1u);
                         }
-                        umma_commit(&sh.dig_empty[dg]);
+                        umma_commit(&sh.dig_empty[rd.s]);
+                        if (k0 + kChunk >= k_pad) {
+                            umma_commit(&sh.acc_full[rt.s]);
+                            if (n == 1) umma_commit(&sh.a_empty[ra.s]);
+                        }
                     }
-                    if (ok) umma_commit(&sh.acc_full[acc]);
+                    __syncwarp();
+                    a0 += 512;
+                    rd.next(a.tc_dig_stages);
                 }
-                if (ok) umma_commit(&sh.a_empty);
+                rt.next(kAccStages);
             }
-            // every MMA issued has completed before TMEM is released
-            umma_commit(&sh.drain);
-            mbar_wait_bounded(&sh.drain, 0, nullptr);
+            ra.next(a.tc_a_stages);
         }
+        // every MMA issued has completed before TMEM is released
+        if (leader) umma_commit(&sh.drain);
+        mbar_wait_bounded(&sh.drain, 0, nullptr);
         __syncwarp();
     } else {
         // ------------------------------------------------------------ epilogue
-        const uint32_t row = warp * 32 + lane;
-        const uint32_t t_lane = (warp * 32) << 16;
-        uint32_t *stage_rows = reinterpret_cast<uint32_t *>(stage_out);
-        uint32_t *srow = stage_rows + row * kOutRow;
-        uint32_t tcount = 0;
+        const uint32_t team = warp / kEpiWarps, quadrant = warp % 4;  // tiles taken, TMEM lanes
+        const uint32_t half = (warp / 4) % 2;                         // columns [32 half, + 32) of the tile
+        const uint32_t row = quadrant * 32 + lane;
+        const uint32_t stage = smem_addr(stage_out + warp * kOutBox);
+        Ring rt;  // accumulator stage of the tile
+        uint32_t turn = 0, lwe_next = 0xFFFFFFFFu;
         bool ok = true;
-        for (uint32_t u = blockIdx.x; ok && u < a.n_units; u += gridDim.x) {
-            const Unit x = unit_of(a, u);
-            const uint32_t o = x.blk.out_lo + row;
-            const bool has = o < x.blk.out_hi && o >= a.out_lo && o < a.out_hi;
-            const uint32_t bias = has ? a.tc_bias[o] : 0u;
+        // the unit's outputs are read two units ahead, this lane's constants one
+        Units head(a);
+        uint32_t lo = 0, hi = 0, next_o = 0;
+        bool next_has = false;
+        TcOut next_oc{};
+        auto fetch_header = [&]() {
+            lo = hi = 0;
+            if (head.valid(a)) {
+                lo = head.header(a)->out_lo;
+                hi = head.header(a)->out_hi;
+            }
+            head.next(a);
+        };
+        auto fetch_constants = [&]() {  // of the block header last read
+            next_o = lo + row;
+            next_has = next_o < hi && next_o >= a.out_lo && next_o < a.out_hi;
+            next_oc = TcOut{0, 0, 0.75f, 0.75f};
+            if (next_has) next_oc = a.tc_out[next_o];
+        };
+        fetch_header();
+        fetch_constants();
+        fetch_header();
+        for (Units w(a); ok && w.valid(a); w.next(a)) {
+            const uint32_t o = next_o;
+            const bool has = next_has;
+            const TcOut oc = next_oc;
+            fetch_constants();
+            fetch_header();
+            const uint32_t add0 = oc.offset - kMagicSum;
             uint8_t *orow = has ? a.out + (a.out_row_map ? uint64_t(a.out_row_map[o]) : uint64_t(o) - a.out_row_base) *
                                               a.out_stride
                                 : nullptr;
-            for (uint32_t sl = x.s0; ok && sl < x.s1; ++sl, ++tcount) {
-                const uint32_t acc = tcount % kAccStages;
-                if (!(ok = tc_warp_wait(&sh.abort, &sh.acc_full[acc], (tcount / kAccStages) & 1u, a.err, lane))) break;
+            // the warp's 32 outputs are all wanted: whole boxes go out
+            const bool boxes = a.tc_store_map && __all_sync(0xFFFFFFFFu, has);
+            const uint32_t s1 = w.s1(a);
+            for (uint32_t sl = w.s0(a); ok && sl < s1; ++sl) {
+                const Ring at = rt;
+                rt.next(kAccStages);
+                const bool mine = turn == team;
+                if (++turn == kEpi) turn = 0;
+                if (!mine) continue;
+                if (!(ok = tc_team_wait<32 * kEpiWarps>(1 + team, warp % kEpiWarps == 0 && lane == 0, &sh.abort,
+                                                        &sh.acc_full[at.s], at.round & 1u, a.err)))
+                    break;
                 tc_fence_after();
-                const uint32_t c0 = sl * kN;
-                const uint32_t valid = min(kN, a.row_words - c0);
-                const bool full = valid == kN;
-                // columns (relative to c0) that take the bias, and that are zeroed
-                uint32_t b_lo = 0, b_hi = 0, z_lo = 0, z_hi = 0;
+                const uint32_t base = tmem + ((quadrant * 32) << 16) + at.s * (4 * kN) + 32 * half;
+                // this warp's 32 columns, from c0; `valid` of them inside the row
+                const uint32_t c0 = sl * kN + 32 * half;
+                const uint32_t valid = c0 < a.row_words ? min(32u, a.row_words - c0) : 0u;
+                // columns that take the bias, and that are zeroed
+                uint32_t bias_cols = 0, zero_cols = 0;
                 if (a.form == kFormTrlwe) {
-                    auto rel = [&](uint32_t c) { return c <= c0 ? 0u : min(c - c0, kN); };
-                    b_lo = rel(a.N);
-                    b_hi = rel(a.N + a.num_samples);
-                    z_lo = rel(a.N + a.region_size);
-                    z_hi = rel(2 * a.N);
+                    bias_cols = columns_in(c0, a.N, a.N + a.num_samples);
+                    zero_cols = columns_in(c0, a.N + a.region_size, 2 * a.N);
                 } else {
-                    const uint32_t first = (a.lwe_n1 - 1u) - c0 % a.lwe_n1;  // next column c with c % n1 == n
-                    b_lo = min(first, kN);
-                    b_hi = min(first + 1u, kN);
+                    // body words: columns c with c % n1 == n; lwe_next is the first from c0 on
+                    if (lwe_next < c0 || lwe_next - c0 >= a.lwe_n1) lwe_next = c0 + (a.lwe_n1 - 1u) - c0 % a.lwe_n1;
+                    for (uint32_t c = lwe_next - c0; c < 32; c += a.lwe_n1) bias_cols |= 1u << c;
                 }
-                // warp-uniform fast path: the bias on every column or none, nothing zeroed
-                const bool uniform = z_lo >= z_hi && (b_lo >= b_hi || (b_lo == 0 && b_hi == kN));
-                const uint32_t add_all = (b_lo == 0 && b_hi == kN ? bias : 0u) - kMagicSum;
-                const uint32_t base = tmem + t_lane + acc * 256;
+                const bool mixed = zero_cols != 0 || (bias_cols != 0 && bias_cols != 0xFFFFFFFFu);
+                const uint32_t add_all = (bias_cols == 0xFFFFFFFFu ? oc.bias : 0u) + add0;
 #pragma unroll
-                for (uint32_t cc = 0; cc < kN / 16; ++cc) {
-                    uint32_t d0[16], d1[16], d2[16], d3[16];
-                    tmem_ld16(base + cc * 16, d0);
-                    tmem_ld16(base + 64 + cc * 16, d1);
-                    tmem_ld16(base + 128 + cc * 16, d2);
-                    tmem_ld16(base + 192 + cc * 16, d3);
-                    tmem_wait_ld();
-                    uint32_t v[16];
+                for (uint32_t cc = 0; cc < 4; ++cc) {
+                    uint32_t d[4][8], v[8];
 #pragma unroll
-                    for (uint32_t j = 0; j < 16; ++j) {
-                        const uint32_t u0 = __float_as_uint(__fadd_rn(__uint_as_float(d0[j]), 12582912.0f));
-                        const uint32_t u1 = __float_as_uint(__fadd_rn(__uint_as_float(d1[j]), 12582912.0f));
-                        const uint32_t u2 = __float_as_uint(__fadd_rn(__uint_as_float(d2[j]), 12582912.0f));
-                        const uint32_t u3 = __float_as_uint(__fadd_rn(__uint_as_float(d3[j]), 12582912.0f));
-                        v[j] = ((u3 * 256u + u2) * 256u + u1) * 256u + u0;
+                    for (uint32_t s = 0; s < 4; ++s) tmem_ld8(base + s * kN + cc * 8, d[s]);
+                    if (cc == 0) {
+                        if (lane == 0) bulk_wait_read<0>();  // the box stored last has been read
+                        __syncwarp();
                     }
-                    if (uniform) {
+                    tmem_wait_ld();
+                    if (cc == 3) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&sh.acc_empty[at.s]);
+                    }
 #pragma unroll
-                        for (uint32_t j = 0; j < 16; ++j) v[j] += add_all;
-                    } else {
+                    for (uint32_t j = 0; j < 8; j += 2) {
+                        add2(d[0][j], d[0][j + 1], oc.m0);
+                        add2(d[1][j], d[1][j + 1], oc.m1);
+                        add2(d[2][j], d[2][j + 1], oc.m1);
+                        add2(d[3][j], d[3][j + 1], oc.m1);
+                    }
 #pragma unroll
-                        for (uint32_t j = 0; j < 16; ++j) {
-                            const uint32_t col = cc * 16 + j;
-                            v[j] += (col >= b_lo && col < b_hi ? bias : 0u) - kMagicSum;
-                            if (col >= z_lo && col < z_hi) v[j] = 0u;
+                    for (uint32_t j = 0; j < 8; ++j)
+                        v[j] = (((d[3][j] << 24) + add_all) + (d[2][j] << 16)) + ((d[1][j] << 8) + d[0][j]);
+                    if (mixed) {
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j) {
+                            const uint32_t bit = 1u << (cc * 8 + j);
+                            if (bias_cols != 0xFFFFFFFFu && (bias_cols & bit)) v[j] += oc.bias;
+                            if (zero_cols & bit) v[j] = 0u;
                         }
                     }
-                    if (full) {
+                    // 16-byte piece p of the box's row goes to piece p ^ (row % 8)
 #pragma unroll
-                        for (uint32_t j = 0; j < 16; j += 4) sts_v4(smem_addr(srow + cc * 16 + j), v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else if (has) {
-                        uint32_t *g = reinterpret_cast<uint32_t *>(orow) + c0 + cc * 16;
-#pragma unroll
-                        for (uint32_t j = 0; j < 16; ++j)
-                            if (cc * 16 + j < valid) g[j] = v[j];
-                    }
+                    for (uint32_t j = 0; j < 8; j += 4)
+                        sts_v4(stage + lane * 128 + ((cc * 2 + j / 4) ^ (lane % 8)) * 16, v[j], v[j + 1], v[j + 2],
+                               v[j + 3]);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh.acc_empty[acc]);
-                if (full) {
-                    // the warp's 32 staged rows, row by row: lanes 0-15 and
-                    // 16-31 each store one row's 256 bytes as coalesced
-                    // 16-byte stores; row r's address comes from lane r
+                if (boxes) {
+                    fence_proxy_async_smem();
                     __syncwarp();
-                    const uint32_t half = lane / 16, q = lane % 16;
-                    const uint64_t mine = reinterpret_cast<uint64_t>(orow);
-#pragma unroll 4
-                    for (uint32_t i = 0; i < 16; ++i) {
-                        const uint32_t r = 2 * i + half;
-                        const uint64_t dst = __shfl_sync(0xFFFFFFFFu, mine, r);
-                        const uint4 w = lds_v4p(stage_rows + (warp * 32 + r) * kOutRow + 4 * q);
-                        if (dst)
-                            stg_cs_v4(reinterpret_cast<uint8_t *>(dst) + uint64_t(c0) * 4 + 16 * q,
-                                      make_int4(int(w.x), int(w.y), int(w.z), int(w.w)));
+                    if (lane == 0 && valid) {
+                        tma_store_2d(&maps.out, int32_t(c0), int32_t(o - uint32_t(a.out_row_base)), stage);
+                        bulk_commit();
                     }
-                    __syncwarp();  // the warp has read its staged rows before the next tile writes them
+                    continue;
                 }
+                __syncwarp();
+                // row by row: eight lanes store 128 bytes of one row, four
+                // rows at a time; row r's address comes from lane r
+                const uint32_t p = lane % 8;
+                const uint64_t mine_row = reinterpret_cast<uint64_t>(orow);
+#pragma unroll 1
+                for (uint32_t i = 0; i < 8; ++i) {
+                    const uint32_t r = 4 * i + lane / 8;
+                    const uint64_t dst = __shfl_sync(0xFFFFFFFFu, mine_row, r);
+                    const uint4 w = lds_v4_ordered(stage + r * 128 + (p ^ (r % 8)) * 16);
+                    if (!dst || 4 * p >= valid) continue;
+                    uint32_t *g = reinterpret_cast<uint32_t *>(dst) + c0 + 4 * p;
+                    if (4 * p + 4 <= valid) {
+                        stg_cs_v4(g, make_int4(int(w.x), int(w.y), int(w.z), int(w.w)));
+                    } else {
+                        g[0] = w.x;
+                        if (4 * p + 1 < valid) g[1] = w.y;
+                        if (4 * p + 2 < valid) g[2] = w.z;
+                    }
+                }
+                __syncwarp();  // the warp has read its staged rows before they are overwritten
             }
         }
+        if (lane == 0) bulk_wait();  // the stored boxes are written
     }
 
     tc_fence_before();
@@ -447,32 +703,36 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
-// The input rows as a 2D tensor (row_words columns x n_rows rows, uint32,
-// row stride in_stride bytes) read in boxes of 68 columns x 32 rows: one
-// chunk of a raw stage.  False when the layout cannot be encoded (the kernel
-// then copies row by row).
-bool encode_rows_map(const ScoreArgs &a, CUtensorMap *map) {
+// A 2D tensor of uint32 (`words` columns x `rows` rows, `stride` bytes between
+// rows) read or written in boxes.  False when it cannot be encoded (the
+// kernel then copies row by row).
+bool encode_rows_map(const uint8_t *base, uint64_t words, uint64_t rows, uint64_t stride, uint32_t box_words,
+                     uint32_t box_rows, CUtensorMapSwizzle swizzle, CUtensorMap *map) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (!enc || a.n_rows == 0 || a.in_stride % 16 || (reinterpret_cast<uintptr_t>(a.in) & 15u)) return false;
-    const cuuint64_t dims[2] = {a.row_words, a.n_rows};
-    const cuuint64_t strides[1] = {a.in_stride};
-    const cuuint32_t box[2] = {kRawRow, kChunk};
+    if (!enc || rows == 0 || rows > 0x7FFFFFFFull || stride % 16 || (reinterpret_cast<uintptr_t>(base) & 15u))
+        return false;
+    const cuuint64_t dims[2] = {words, rows};
+    const cuuint64_t strides[1] = {stride};
+    const cuuint32_t box[2] = {box_words, box_rows};
     const cuuint32_t elem[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(a.in), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(base), dims, strides, box, elem,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace
 
 size_t tc_smem_bytes(uint32_t max_k_pad) {
-    const size_t need = kHeader + size_t(tc_a_bytes(max_k_pad)) + size_t(kRawStages) * kRawStageBytes +
-                        size_t(kDigStages) * kDigStageBytes + kOutBytes;
-    return need < kMinSmem ? kMinSmem : need;
+    const TcShape *x = tc_shape(max_k_pad);
+    return x ? x->smem(max_k_pad) : SIZE_MAX;
 }
 
 cudaError_t configure_tc_kernel(size_t max_smem) {
-    return cudaFuncSetAttribute(k_score_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(max_smem));
+    for (auto *fn : {k_score_tc<2, 2, 2>, k_score_tc<1, 3, 4>}) {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(max_smem));
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_score_tc(const ScoreArgs &a_in, uint32_t ctas, cudaStream_t stream) {
@@ -480,12 +740,26 @@ cudaError_t launch_score_tc(const ScoreArgs &a_in, uint32_t ctas, cudaStream_t s
     if (a_in.accumulate || a_in.digest || a_in.units_per_block == 0 || a_in.unit_slices == 0)
         return cudaErrorInvalidValue;
     ScoreArgs a = a_in;
-    CUtensorMap map;
-    std::memset(&map, 0, sizeof(map));
-    a.tc_use_map = encode_rows_map(a, &map) ? 1u : 0u;
-    const size_t smem = tc_smem_bytes(a.tc_a_max_bytes / uint32_t(tc_a_bytes(1)));
+    const uint32_t k = a.tc_a_max_bytes / uint32_t(tc_a_bytes(1));
+    const TcShape *shape = tc_shape(k);
+    if (!shape) return cudaErrorInvalidValue;
+    a.tc_a_stages = shape->a_stages;
+    a.tc_dig_stages = shape->dig_stages;
+    a.tc_raw_stages = shape->raw_stages;
+    TcMaps maps;
+    std::memset(&maps, 0, sizeof(maps));
+    a.tc_use_map = encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, kChunk, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                   &maps.rows) &&
+                   encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, 1, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                   &maps.gather);
+    a.tc_store_map = !a.out_row_map && a.out_lo >= a.out_row_base &&
+                     encode_rows_map(a.out, a.row_words, a.out_hi - a.out_row_base, a.out_stride, 32, 32,
+                                     CU_TENSOR_MAP_SWIZZLE_128B, &maps.out);
     const uint32_t grid = ctas < a.n_units ? ctas : a.n_units;
-    k_score_tc<<<grid, kThreads, smem, stream>>>(a, map);
+    a.unit_step_blocks = grid / a.units_per_block;
+    a.unit_step_parts = grid % a.units_per_block;
+    auto *fn = shape->epi == 2 ? k_score_tc<2, 2, 2> : k_score_tc<1, 3, 4>;
+    fn<<<grid, tc_threads(shape->epi, shape->conv, shape->conv_warps), shape->smem(k), stream>>>(a, maps);
     return cudaGetLastError();
 }
 

@@ -37,6 +37,16 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
                  : "memory");
 }
 
+// One thread of the (converged) warp.  The issuing warp runs its loop whole
+// and branches on this around the MMAs only: the descriptors then stay in
+// uniform registers.  With the loop under `lane == 0` a chunk of four MMAs of
+// 448 tensor cycles took 538 to 685 cycles to issue, this way 453 to 483.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+
 // One warp: allocates `cols` TMEM columns, their address into *slot (shared).
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)), "r"(cols)
@@ -68,7 +78,12 @@ __device__ __forceinline__ bool tc_wait(uint32_t *abort, uint64_t *bar, uint32_t
     if (mbar_try_wait(bar, parity)) return true;
     volatile uint32_t *flag = abort;
     const long long t0 = clock64();
-    while (!mbar_try_wait_sleep(bar, parity, 20000u)) {
+    for (;;) {
+        // a few tries between looks at the flag and the clock: waiting warps
+        // share the issue slots with working ones
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i)
+            if (mbar_try_wait_sleep(bar, parity, 20000u)) return true;
         if (*flag != 0) return false;
         if (clock64() - t0 > kWaitLimitCycles) {
             report_error(err, kDevTimeout);
@@ -76,7 +91,6 @@ __device__ __forceinline__ bool tc_wait(uint32_t *abort, uint64_t *bar, uint32_t
             return false;
         }
     }
-    return true;
 }
 
 // Lane 0 waits, the warp follows its verdict.
@@ -85,6 +99,30 @@ __device__ __forceinline__ bool tc_warp_wait(uint32_t *abort, uint64_t *bar, uin
     uint32_t ok = 1;
     if (lane == 0) ok = tc_wait(abort, bar, parity, err) ? 1u : 0u;
     return __shfl_sync(0xFFFFFFFFu, ok, 0) != 0;
+}
+
+// Whether `ok` holds for all kThreads threads of a team of warps, at named
+// barrier `id` (1 .. 15).  A team waits with one thread polling and the others
+// standing here, where they take no issue slots.  (Every warp polling for
+// itself made up half of the instructions that the scoring kernel issued.)
+template <int kThreads>
+__device__ __forceinline__ bool tc_team_and(uint32_t id, bool ok) {
+    uint32_t r = ok ? 1u : 0u;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %0, 0;\n\t"
+        "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "+r"(r)
+        : "r"(id), "n"(kThreads)
+        : "memory");
+    return r != 0;
+}
+
+template <int kThreads>
+__device__ __forceinline__ bool tc_team_wait(uint32_t id, bool polls, uint32_t *abort, uint64_t *bar, uint32_t parity,
+                                             uint32_t *err) {
+    return tc_team_and<kThreads>(id, !polls || tc_wait(abort, bar, parity, err));
 }
 
 }  // namespace idash
