@@ -218,6 +218,7 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
         // are loaded once per unit
         a.tc_a = m->d_tc_a;
         a.tc_out = m->d_tc_out;
+        a.tc_producers = m->plan.tc_producers;
         a.tc_a_max_bytes = uint32_t(tc_a_bytes(m->max_terms));
         const uint64_t tiles = uint64_t(a.n_blocks) * a.n_slices;
         const uint64_t want = std::max<uint64_t>(1, uint64_t(m->ctas) * 32);

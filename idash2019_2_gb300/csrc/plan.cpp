@@ -350,6 +350,7 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
     }
     plan->phase_begin.push_back(0);
     std::vector<uint64_t> win, merged;
+    uint64_t chunks = 0, scattered = 0;
     for (uint64_t o = 0; o < n_out;) {
         win.clear();
         uint64_t e = o;
@@ -379,6 +380,8 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
             bool run = true;
             for (size_t k = c0 + 1; k < c1 && run; ++k) run = (win[k] >> 32) == (win[c0] >> 32) + (k - c0);
             if (run && c < 32) b.term_begin |= 1u << c;
+            ++chunks;
+            scattered += !run;
         }
         b.n_terms = uint32_t(nm.nptr[e] - nm.nptr[o]);
         b.out_lo = uint32_t(o);
@@ -414,6 +417,7 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         plan->blocks.push_back(b);
         o = e;
     }
+    plan->tc_producers = 4 * scattered > chunks ? kTcMaxProducers : 1;
     plan->phase_begin.push_back(uint32_t(plan->blocks.size()));
     return "";
 }

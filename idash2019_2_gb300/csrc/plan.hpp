@@ -112,6 +112,7 @@ struct Plan {
     // digits in the MMA's shared-memory layout, and every output's constants.
     std::vector<uint8_t> tc_a;
     std::vector<TcOut> tc_out;
+    uint32_t tc_producers = 1;  // kTcMaxProducers where more than a quarter of the 32-row chunks are scattered rows
 };
 
 // Tensor-core plans (build_tc_plan).  A block is up to kTcRows consecutive
@@ -133,6 +134,10 @@ struct Plan {
 // 0.75 * 2^24 stays in one binade (score_tc.cu).  It refuses models with a
 // coefficient outside two digits.
 constexpr uint32_t kTcRows = 128;
+// The second row-loading warp is worth it where rows are copied one by one
+// (10 neighbours over permuted rows: one 0.327 ms, two 0.261) and not where a
+// chunk is one tensor copy (5 neighbours, consecutive rows: 0.421 and 0.430).
+constexpr uint32_t kTcMaxProducers = 2;
 constexpr uint32_t kTcMaxK = 192;  // shared-memory bound on the padded K
 struct TcLimits {
     uint32_t max_k = kTcMaxK;

@@ -71,6 +71,7 @@ struct ScoreArgs {
     const TcOut *tc_out;
     uint32_t unit_slices, units_per_block, n_units;
     uint32_t tc_a_max_bytes;      // shared-memory room for one block's digits
+    uint32_t tc_producers;        // row-loading warps (Plan::tc_producers)
     uint32_t unit_step_blocks, unit_step_parts;  // set by the launch: gridDim.x units in blocks and units of a block
     uint32_t tc_use_map, tc_store_map;  // set by the launch: rows come, and outputs go, by tensor copies
     uint32_t tc_a_stages, tc_dig_stages, tc_raw_stages;  // set by the launch: buffers of each kind

@@ -21,30 +21,36 @@
 // the balanced sum, in [0.5, 1), where the last place is 2^-24 and the bits
 // are an integer; the plan's per-output constant puts 128 S_s back.
 //
-// Structure (one CTA of 23 warps per SM, persistent over work units of
-// (block, run of 64-column slices)); each role's hand-offs take hundreds of
-// cycles, so the roles that would otherwise be bound by them come in teams
-// that take tiles or chunks in turn:
-//   warp 12     producer: per chunk of 32 rows, the rows' 64-column slices: one
-//               2D tensor copy when the chunk's rows are consecutive, else
-//               eight four-row gathers;
-//   warp 14     loads the block's coefficient digits (one bulk copy, kept in
-//               shared memory for the unit, the next unit's beside them where
-//               they fit);
-//   warps 15-22 converters, two teams of four for every other chunk: eight
-//               rows of a column -> one 16-byte row of each of the four byte
-//               planes, in the MMA's no-swizzle K-major layout with the
-//               planes side by side along N;
-//   warp 13     allocates the 512 TMEM columns and issues two tcgen05.mma
-//               per K = 16 step (M = 128: c0 times the four planes, N = 256,
-//               and c1 times the first three, N = 192, one accumulator to the
-//               right) into a double-buffered set of four fp32 accumulators;
-//   warps 0-11  epilogue, three teams of four for every third tile:
-//               tcgen05.ld of the accumulators (a warp reads 32 TMEM lanes,
-//               one output each), the digit recombination, bias and zeroed
-//               columns, staged in shared memory (128-byte swizzle) and
-//               stored by 2D tensor copies of 32 rows x 32 columns, or row by
-//               row where the 32 rows are not all wanted or not consecutive.
+// Structure (one persistent CTA per SM over work units of (block, run of
+// 64-column slices)).  A role's hand-offs and lookups take hundreds of
+// cycles, as long as the work itself on a tile, so the roles that would bound
+// the kernel come in teams that take tiles or chunks in turn:
+//   producers   (one or two warps) per chunk of 32 rows, the rows' 64-column
+//               slices: one 2D tensor copy when the chunk's rows are
+//               consecutive, else 16-byte copies, two rows per instruction;
+//   digits      (one warp) loads the block's coefficient digits (one bulk
+//               copy, kept in shared memory for the unit, the next unit's
+//               beside them where they fit);
+//   converters  (two teams of two warps or three of four) eight rows of a
+//               column -> one 16-byte row of each of the four byte planes, in
+//               the MMA's no-swizzle K-major layout with the planes side by
+//               side along N;
+//   MMA         (one warp) owns the 512 TMEM columns and issues two
+//               tcgen05.mma per K = 16 step (M = 128: c0 times the four
+//               planes, N = 256, and c1 times the first three, N = 192, one
+//               accumulator to the right) into a double-buffered set of four
+//               fp32 accumulators;
+//   epilogue    (one or two teams of eight warps) tcgen05.ld of the
+//               accumulators (a warp reads 32 TMEM lanes, one output each,
+//               and half the columns), the digit recombination, bias and
+//               zeroed columns, staged in shared memory (128-byte swizzle)
+//               and stored by 2D tensor copies of 32 rows x 32 columns, or
+//               row by row where the 32 rows are not all wanted or not
+//               consecutive.
+// What bounds it, and what it measured: 5 neighbours (K = 64, 2.4 GB) the
+// roles' instructions, about 5200 a tile: 0.42 ms against 0.36 ms of memory
+// traffic; 30 neighbours (K = 192) the conversion and the MMAs, 448 cycles of
+// MMA per 32 rows.
 // Every wait is bounded; a wait that expires records IDASH_ERR_DEVICE_TIMEOUT,
 // raises a CTA-wide abort flag that ends the other roles' waits, and each
 // role then waits (bounded) for its own copies and MMAs in flight before the
@@ -74,15 +80,15 @@ constexpr uint32_t kRawStageBytes = kChunk * kN * 4;
 constexpr uint32_t kGroupBytes = 4 * kN * 16;           // 8 rows of the four planes
 constexpr uint32_t kDigStageBytes = (kChunk / 8) * kGroupBytes;
 constexpr uint32_t kOutBox = 32 * 32 * 4;               // one stored box: 32 rows x 32 columns
-constexpr uint32_t kHeader = 1024;
-// Warps: kEpi teams of eight (one, or one per accumulator stage), then one
-// each of producer, MMA and digit loads, then kConv converter teams of
+constexpr uint32_t kHeader = 2048;
+// Warps: kEpi teams of eight (one, or one per accumulator stage), kProducers
+// producers, one each of MMA and digit loads, then kConv converter teams of
 // kConvWarps.  A parity tells only two successive phases of a barrier apart,
 // so a team must meet all phases of the stages it waits for in turn: a stage
 // belongs to one team.
 constexpr uint32_t kEpiWarps = 8;
-constexpr uint32_t tc_threads(uint32_t epi, uint32_t conv, uint32_t conv_warps) {
-    return 32 * (kEpiWarps * epi + 3 + conv_warps * conv);
+constexpr uint32_t tc_threads(uint32_t epi, uint32_t conv, uint32_t conv_warps, uint32_t producers) {
+    return 32 * (kEpiWarps * epi + producers + 2 + conv_warps * conv);
 }
 constexpr uint32_t kTmemCols = 512;                     // 2 stages x 4 accumulators x 64 columns
 constexpr uint32_t kIdescAll = umma_idesc_f16(kM, 4 * kN), kIdescHigh = umma_idesc_f16(kM, 3 * kN);
@@ -92,10 +98,15 @@ constexpr uint32_t kMagicSum = kMagic + (kMagic << 8) + (kMagic << 16) + (kMagic
 constexpr size_t kMinSmem = 120 * 1024;
 constexpr size_t kMaxSmem = 227 * 1024;
 
-// Teams and buffers for a plan whose largest padded K is k.  Small K: the
-// epilogue is most of the work (two teams, one per accumulator stage); large
-// K: the conversion is.  Then the first set of buffers that fits.  Raw and
-// digit stages are multiples of the converter teams (see above).
+// Teams and buffers for a plan whose largest padded K is k: the first that
+// fits.  Small K: the epilogue is most of the work (two teams, one per
+// accumulator stage) and copies in flight cover the memory's latency (eight
+// raw stages up to K = 64, six up to 80).  Large K: the conversion is (three
+// teams of four warps).  42,000 outputs over 2,100 rows, first and second
+// kind: K = 48 0.101 and 0.117 ms, K = 80 0.114 and 0.123, K = 96 0.126 and
+// 0.122; 6,000 outputs, K = 128 to 160: 0.076 to 0.090 and 0.071 to 0.081.
+// Raw and digit stages are multiples of the converter teams (see above), raw
+// stages of the producers too.
 struct TcShape {
     uint32_t epi, conv, conv_warps;
     uint32_t a_stages;    // blocks' coefficient digits
@@ -107,8 +118,7 @@ struct TcShape {
         return n < kMinSmem ? kMinSmem : n;
     }
 };
-constexpr TcShape kTcShapes[] = {{2, 2, 2, 2, 4, 6}, {2, 2, 2, 2, 4, 4}, {2, 2, 2, 1, 4, 6}, {2, 2, 2, 1, 4, 4},
-                                 {1, 3, 4, 1, 3, 6}};
+constexpr TcShape kTcShapes[] = {{2, 2, 2, 2, 2, 8}, {2, 2, 2, 2, 2, 6}, {1, 3, 4, 2, 3, 6}, {1, 3, 4, 1, 3, 6}};
 const TcShape *tc_shape(uint32_t k) {
     for (const TcShape &x : kTcShapes)
         if (x.smem(k) <= kMaxSmem) return &x;
@@ -122,8 +132,9 @@ struct TcBars {
     uint64_t acc_full[kAccStages], acc_empty[kAccStages];
     uint32_t tmem_base;
     uint32_t abort;
+    uint32_t rows[kTcMaxProducers][kTcMaxK];  // the unit's input rows, per producer
 };
-static_assert(sizeof(TcBars) <= kHeader, "barrier area");
+static_assert(sizeof(TcBars) <= kHeader, "header area");
 
 // A position in a ring of n stages; parity of the round.
 struct Ring {
@@ -161,11 +172,6 @@ __device__ __forceinline__ void add2(uint32_t &x, uint32_t &y, float m) {
         : "f"(m));
 }
 
-__device__ __forceinline__ void expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-
 // 2D tensor copy of the box at (x = column, y = row) into shared memory,
 // completed on `bar` as transaction bytes.  x * 4 is a multiple of 16.
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int32_t x, int32_t y, uint64_t *bar) {
@@ -176,14 +182,14 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-// Four rows' boxes (one row high) at column x, one after another in shared memory.
-__device__ __forceinline__ void tma_gather4(void *dst, const CUtensorMap *map, int32_t x, const int32_t (&y)[4],
-                                            uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
-        "%3, %4, %5, %6}], [%7];" ::"r"(smem_addr(dst)),
-        "l"(map), "r"(x), "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(smem_addr(bar))
-        : "memory");
+// 16 bytes global -> shared (zeros when `bytes` is 0), counted by the
+// cp_async_arrive that follows it.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// `bar`'s phase also waits for this thread's cp.async so far.
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.shared.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int32_t x, int32_t y, uint32_t src) {
@@ -246,48 +252,35 @@ __device__ __forceinline__ uint32_t columns_in(uint32_t c0, uint32_t lo, uint32_
     return from < to ? (0xFFFFFFFFu >> (32u - (to - from))) << from : 0u;
 }
 
-// The launch's tensor maps: rows (boxes of 64 columns x 32 rows), row
-// gathers (64 x 1) and outputs (32 x 32, 128-byte swizzle).
+// The launch's tensor maps: rows (boxes of 64 columns x 32 rows) and outputs
+// (32 x 32, 128-byte swizzle).
 struct TcMaps {
-    CUtensorMap rows, gather, out;
+    CUtensorMap rows, out;
 };
 
-// n (at most 32) rows that one box does not hold, slots slot .. slot + n - 1,
-// into a raw stage: four-row gathers, or one copy per row where the launch has
-// no tensor maps.  The whole warp calls it.
-__device__ __noinline__ void load_rows(const ScoreArgs &a, const CUtensorMap &gather, uint32_t slot, uint32_t n,
-                                       uint32_t c0, uint8_t *dst, uint64_t *full, uint32_t lane) {
-    // the row of slot i (the last ones repeated), 0 for one outside the input
-    auto row_of = [&](uint32_t i) {
-        const uint32_t r = a.slots[slot + min(i, n - 1)].row - a.row_base;
-        if (r < a.n_rows) return r;
-        report_error(a.err, kDevBadIndex);
-        return 0u;
-    };
-    fence_proxy_async_smem();  // after the converters' reads of the stage
-    if (n && a.n_rows) {
-        if (a.tc_use_map) {
-            if (4 * lane < n) {
-                const int32_t y[4] = {int32_t(row_of(4 * lane)), int32_t(row_of(4 * lane + 1)),
-                                      int32_t(row_of(4 * lane + 2)), int32_t(row_of(4 * lane + 3))};
-                expect_tx(full, 4 * kN * 4);
-                tma_gather4(dst + lane * (4 * kN * 4), &gather, int32_t(c0), y, full);
-            }
-        } else if (lane < n) {
-            const uint32_t bytes = ((min(kN, a.row_words - c0) + 3u) & ~3u) * 4u;
-            const uint32_t r = row_of(lane);
-            expect_tx(full, bytes);
-            bulk_g2s(dst + lane * (kN * 4), a.in + uint64_t(r) * a.in_stride + uint64_t(c0) * 4, bytes, full);
-        }
-    }
+// n rows of a chunk that one box does not hold into a raw stage, two rows per
+// instruction.  The whole warp calls it.  (Four-row tensor gathers took 270
+// cycles each: 10 neighbours over permuted rows 0.324 ms with them, 0.309 ms
+// this way.)
+__device__ __forceinline__ void load_rows(const ScoreArgs &a, const uint32_t *rows, uint32_t n, uint32_t c0,
+                                          uint32_t dst, uint64_t *full, uint32_t lane) {
+    const uint32_t half = lane / 16, word = c0 + 4 * (lane % 16);
+    const uint32_t bytes = word < a.row_words ? 16u : 0u;  // rows are whole 16-byte pieces apart
+    const uint8_t *src = a.in + uint64_t(bytes ? word : 0u) * 4;
+    dst += half * (kN * 4) + (lane % 16) * 16;
+#pragma unroll 4
+    for (uint32_t i = 0; i < n; i += 2)
+        cp_async16(dst + i * (kN * 4), src + uint64_t(rows[min(i + half, n - 1)]) * a.in_stride, bytes);
+    cp_async_arrive(full);
     __syncwarp();
     if (lane == 0) mbar_arrive(full);
 }
 
-template <uint32_t kEpi, uint32_t kConv, uint32_t kConvWarps>
-__global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps), 1)
+template <uint32_t kEpi, uint32_t kConv, uint32_t kConvWarps, uint32_t kProducers>
+__global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers), 1)
     k_score_tc(const __grid_constant__ ScoreArgs a, const __grid_constant__ TcMaps maps) {
-    constexpr uint32_t kProducerWarp = kEpiWarps * kEpi, kMmaWarp = kProducerWarp + 1, kDigitWarp = kMmaWarp + 1;
+    constexpr uint32_t kProducerWarp = kEpiWarps * kEpi, kMmaWarp = kProducerWarp + kProducers;
+    constexpr uint32_t kDigitWarp = kMmaWarp + 1;
     constexpr uint32_t kConvWarp0 = kDigitWarp + 1;
     extern __shared__ __align__(1024) uint8_t smem[];
     TcBars &sh = *reinterpret_cast<TcBars *>(smem);
@@ -346,16 +339,23 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps), 1)
             }
         }
         __syncwarp();
-    } else if (warp == kProducerWarp) {
+    } else if (warp >= kProducerWarp && warp < kMmaWarp) {
         // ------------------------------------------------------------ producer
         // The block header is read two units ahead and the rows one unit
         // ahead, so that the loop below issues copies and nothing else: with
         // the lookups in it, it took 850 cycles per chunk and bound the kernel.
         struct Rows {
-            uint32_t n_slots, slot_begin, runs, n_chunks;  // runs: the block's consecutive-chunk mask
-            uint32_t first;                                // lane c: first row of chunk c
+            uint32_t n_slots, runs, n_chunks;  // runs: the block's consecutive-chunk mask
+            uint32_t row[kMaxChunks];          // lane i: row i of each chunk
         };
         const bool leader = elect_one();
+        // Each of the producers takes its chunks in turn (the raw stages are a
+        // multiple of both counts).  Copying rows one by one is worth the
+        // second (10 neighbours over permuted rows: one 0.327, two 0.261 ms);
+        // boxes are not (headline 0.421 and 0.430 ms).
+        const uint32_t me = warp - kProducerWarp;
+        uint32_t *rows = sh.rows[me];
+        uint32_t turn = 0;
         Units head(a);
         PlanBlock blk{};
         Rows next{};
@@ -364,32 +364,52 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps), 1)
             head.next(a);
         };
         auto fetch_rows = [&]() {  // of the block header last read
-            next = Rows{blk.n_slots, blk.slot_begin, blk.term_begin, (blk.n_groups + kChunk - 1) / kChunk, 0};
-            if (kChunk * lane < next.n_slots) next.first = a.slots[next.slot_begin + kChunk * lane].row - a.row_base;
+            next.n_slots = blk.n_slots;
+            next.runs = blk.term_begin;
+            next.n_chunks = (blk.n_groups + kChunk - 1) / kChunk;
+#pragma unroll
+            for (uint32_t c = 0; c < kMaxChunks; ++c)
+                if (kChunk * c + lane < blk.n_slots) next.row[c] = a.slots[blk.slot_begin + kChunk * c + lane].row;
         };
         fetch_header();
         fetch_rows();
         fetch_header();
-        Ring rr;
-        uint32_t rc = 0;
-        bool ok = true;
+        Ring rr, last;
+        bool ok = true, any = false;
         for (Units w(a); ok && w.valid(a); w.next(a)) {
             const Rows x = next;
             fetch_rows();
             fetch_header();
-            // chunks that one tensor copy loads: consecutive rows, all inside the input
-            const uint32_t here = kChunk * lane < x.n_slots ? min(kChunk, x.n_slots - kChunk * lane) : 0u;
-            const uint32_t boxes = __ballot_sync(0xFFFFFFFFu, here && a.tc_use_map && ((x.runs >> lane) & 1u) &&
-                                                                  x.first < a.n_rows && here <= a.n_rows - x.first);
-            uint32_t r0[kMaxChunks];
+            // rows as held at a.in; 0, reported, for one outside it
+            __syncwarp();
 #pragma unroll
-            for (uint32_t c = 0; c < kMaxChunks; ++c) r0[c] = __shfl_sync(0xFFFFFFFFu, x.first, c);
+            for (uint32_t c = 0; c < kMaxChunks; ++c) {
+                uint32_t r = x.row[c] - a.row_base;
+                if (kChunk * c + lane < x.n_slots && r >= a.n_rows) {
+                    report_error(a.err, kDevBadIndex);
+                    r = 0;
+                }
+                rows[kChunk * c + lane] = r;
+            }
+            __syncwarp();
+            // lane c: the first row of chunk c; the chunks that one tensor copy
+            // loads (consecutive rows, all inside the input)
+            const uint32_t first = rows[kChunk * min(lane, kMaxChunks - 1)];
+            const uint32_t n_here = kChunk * lane < x.n_slots ? min(kChunk, x.n_slots - kChunk * lane) : 0u;
+            const uint32_t boxes = __ballot_sync(0xFFFFFFFFu, n_here && a.tc_use_map && ((x.runs >> lane) & 1u) &&
+                                                                  first < a.n_rows && n_here <= a.n_rows - first);
             const uint32_t s1 = w.s1(a);
             for (uint32_t sl = w.s0(a); ok && sl < s1; ++sl) {
                 const uint32_t c0 = sl * kN;
-#pragma unroll
-                for (uint32_t c = 0; c < kMaxChunks; ++c) {
-                    if (c >= x.n_chunks) break;
+#pragma unroll 1
+                for (uint32_t c = 0; c < x.n_chunks; ++c) {
+                    const bool mine = turn == me;
+                    if (++turn == kProducers) turn = 0;
+                    if (!mine) {
+                        rr.next(a.tc_raw_stages);
+                        continue;
+                    }
+                    const int32_t r0 = int32_t(__shfl_sync(0xFFFFFFFFu, first, c));
                     uint64_t *full = &sh.raw_full[rr.s];
                     uint8_t *dst = raw + rr.s * kRawStageBytes;
                     if (rr.round > 0 && !(ok = tc_wait(&sh.abort, &sh.raw_empty[rr.s], (rr.round - 1) & 1u, a.err)))
@@ -398,27 +418,29 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps), 1)
                         if (leader) {
                             fence_proxy_async_smem();  // after the converters' reads of the stage
                             mbar_arrive_expect_tx(full, kRawStageBytes);
-                            tma_load_2d(dst, &maps.rows, int32_t(c0), int32_t(r0[c]), full);
+                            tma_load_2d(dst, &maps.rows, int32_t(c0), r0, full);
                         }
-                    } else {
-                        load_rows(a, maps.gather, x.slot_begin + kChunk * c,
-                                  x.n_slots > kChunk * c ? min(kChunk, x.n_slots - kChunk * c) : 0u, c0, dst, full,
-                                  lane);
+                    } else if (x.n_slots > kChunk * c) {
+                        load_rows(a, rows + kChunk * c, min(kChunk, x.n_slots - kChunk * c), c0, smem_addr(dst), full, lane);
+                    } else if (leader) {
+                        mbar_arrive(full);  // rows of padding only: their coefficients are zero
                     }
                     __syncwarp();
-                    ++rc;
+                    last = rr;
+                    any = true;
                     rr.next(a.tc_raw_stages);
                 }
             }
         }
-        // let every copy this CTA issued land: the last fill of each raw
-        // stage (immediate when nothing aborted)
-        if (lane == 0) {
-            for (uint32_t k = 1; k <= a.tc_raw_stages && k <= rc; ++k) {
-                const uint32_t j = rc - k;
-                mbar_wait_bounded(&sh.raw_full[j % a.tc_raw_stages], (j / a.tc_raw_stages) & 1u, nullptr);
+        // Let the copies land: this warp's last ones (immediate when nothing
+        // aborted; every earlier one was waited for by way of its stage's
+        // converters or is behind one of these).
+        if (lane == 0)
+            for (uint32_t s = me; s < a.tc_raw_stages; s += kProducers) {
+                // the stage's last phase that this warp filled
+                const uint32_t filled = last.round + (s <= last.s ? 1u : 0u);
+                if (any && filled) mbar_wait_bounded(&sh.raw_full[s], (filled - 1) & 1u, nullptr);
             }
-        }
         __syncwarp();
     } else if (warp >= kConvWarp0) {
         // ---------------------------------------------------------- converters
@@ -728,7 +750,7 @@ size_t tc_smem_bytes(uint32_t max_k_pad) {
 }
 
 cudaError_t configure_tc_kernel(size_t max_smem) {
-    for (auto *fn : {k_score_tc<2, 2, 2>, k_score_tc<1, 3, 4>}) {
+    for (auto *fn : {k_score_tc<2, 2, 2, 1>, k_score_tc<2, 2, 2, 2>, k_score_tc<1, 3, 4, 1>, k_score_tc<1, 3, 4, 2>}) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(max_smem));
         if (e != cudaSuccess) return e;
     }
@@ -746,20 +768,21 @@ cudaError_t launch_score_tc(const ScoreArgs &a_in, uint32_t ctas, cudaStream_t s
     a.tc_a_stages = shape->a_stages;
     a.tc_dig_stages = shape->dig_stages;
     a.tc_raw_stages = shape->raw_stages;
+    if (a.tc_producers == 0 || a.tc_producers > kTcMaxProducers) return cudaErrorInvalidValue;
     TcMaps maps;
     std::memset(&maps, 0, sizeof(maps));
     a.tc_use_map = encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, kChunk, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                   &maps.rows) &&
-                   encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, 1, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                   &maps.gather);
+                                   &maps.rows);
     a.tc_store_map = !a.out_row_map && a.out_lo >= a.out_row_base &&
                      encode_rows_map(a.out, a.row_words, a.out_hi - a.out_row_base, a.out_stride, 32, 32,
                                      CU_TENSOR_MAP_SWIZZLE_128B, &maps.out);
     const uint32_t grid = ctas < a.n_units ? ctas : a.n_units;
     a.unit_step_blocks = grid / a.units_per_block;
     a.unit_step_parts = grid % a.units_per_block;
-    auto *fn = shape->epi == 2 ? k_score_tc<2, 2, 2> : k_score_tc<1, 3, 4>;
-    fn<<<grid, tc_threads(shape->epi, shape->conv, shape->conv_warps), shape->smem(k), stream>>>(a, maps);
+    const bool two = a.tc_producers == 2;
+    auto *fn = shape->epi == 2 ? (two ? k_score_tc<2, 2, 2, 2> : k_score_tc<2, 2, 2, 1>)
+                               : (two ? k_score_tc<1, 3, 4, 2> : k_score_tc<1, 3, 4, 1>);
+    fn<<<grid, tc_threads(shape->epi, shape->conv, shape->conv_warps, a.tc_producers), shape->smem(k), stream>>>(a, maps);
     return cudaGetLastError();
 }
 
