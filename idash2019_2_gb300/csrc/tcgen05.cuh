@@ -1,6 +1,6 @@
 // tcgen05 and TMEM helpers shared by the tensor-core kernels (score_tc.cu,
-// key_product.cu): descriptors, issue, commit, fences, accumulator loads and
-// the bounded waits of their roles.
+// key_product.cu): descriptors, issue, commit, fences, accumulator loads; and
+// the bounded waits of roles that share a CTA (also intpoly.cu).
 #pragma once
 
 #include "common.cuh"
