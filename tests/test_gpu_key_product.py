@@ -1,7 +1,7 @@
 """The tensor-core product of masks with a binary key (csrc/key_product.cu)
 behind decryption, word for word against the oracle at the edges of its tiles:
-40 rows per item, 16-, 48- and 512-column steps, more row tiles than SMs, rows
-that are only 4-byte aligned, and the largest digit sums."""
+rows per item, columns per load, step and pair of tiles, more row tiles than
+SMs, rows that are only 4-byte aligned, and the largest digit sums."""
 import numpy as np
 import pytest
 
@@ -33,6 +33,7 @@ def _check(ctx, oracle, rows, key, ns, shift=0):
 
 @pytest.mark.parametrize("N,n_rows,ns,shift", [
     (64, 1, 64, 0), (128, 41, 33, 0), (512, 80, 47, 4), (1024, 39, 48, 0), (1024, 40, 49, 8), (1024, 1, 513, 0),
+    (1024, 32, 257, 0), (1024, 33, 31, 0), (512, 31, 512, 0), (2048, 64, 769, 0), (64, 5000, 3, 4),
     (1024, 6121, 100, 0), (1024, 3200, 1000, 4), (2048, 83, 2048, 0), (2048, 1, 1025, 12)])
 def test_tile_edges(ctx, oracle, N, n_rows, ns, shift):
     rng = np.random.default_rng(N + n_rows + ns)
