@@ -161,7 +161,7 @@ idash_status upload_plan(idash_model *m, const Candidate &c, BuiltPlan &&b) {
     m->max_groups = m->plan.max_block_groups;
     uint32_t cps = c.cps;
     if (c.kind == KernelKind::kTc) {
-        if (tc_smem_bytes(m->max_terms) > ctx->smem_optin)
+        if (tc_smem_bytes(m->max_terms, m->plan.tc_rot_bytes != 0) > ctx->smem_optin)
             return ctx->fail(IDASH_ERR_UNSUPPORTED, "tensor-core plan needs more shared memory than a CTA has");
         cps = 1;  // one CTA per SM: it owns the SM's tensor memory
     } else if (c.kind != KernelKind::kDirect) {
@@ -219,6 +219,12 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
         a.tc_a = m->d_tc_a;
         a.tc_out = m->d_tc_out;
         a.tc_producers = m->plan.tc_producers;
+        a.tc_rot_bytes = m->plan.tc_rot_bytes;
+        if (a.tc_rot_bytes) {  // several regions to a row: most of b is zeros
+            const uint32_t live = (m->tp.N + m->tp.region_size + m->slice_words - 1) / m->slice_words;
+            a.zero_slices = a.n_slices > live ? a.n_slices - live : 0;
+            a.n_slices -= a.zero_slices;
+        }
         a.tc_a_max_bytes = uint32_t(tc_a_bytes(m->max_terms));
         const uint64_t tiles = uint64_t(a.n_blocks) * a.n_slices;
         const uint64_t want = std::max<uint64_t>(1, uint64_t(m->ctas) * 32);
@@ -226,6 +232,7 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
         a.units_per_block = (a.n_slices + a.unit_slices - 1) / a.unit_slices;
         a.unit_slices = (a.n_slices + a.units_per_block - 1) / a.units_per_block;  // evenly
         a.n_units = a.n_blocks * a.units_per_block;
+        a.zero_per_unit = (a.zero_slices + a.units_per_block - 1) / a.units_per_block;
     }
     return a;
 }
@@ -365,10 +372,10 @@ std::vector<Candidate> candidates(idash_model *m) {
     std::vector<uint32_t> cpss;
     if (ctx->opt_ctas_per_sm > 0) cpss.push_back(uint32_t(ctx->opt_ctas_per_sm));
     else cpss = {1, 2};
-    // the tensor-core kernel first: exact digit products on tcgen05 (TRLWE
-    // with NUM_REGIONS = 1, and the LWE form), 64-column slices, K up to 192
+    // the tensor-core kernel first: exact digit products on tcgen05, 64-column
+    // slices, K up to 192
     if ((ctx->opt_kernel == 0 || ctx->opt_kernel == 5) && (ctx->opt_slice_words == 0 || ctx->opt_slice_words == 64) &&
-        (m->form == Form::kLwe || (m->form == Form::kTrlwe && m->tp.num_regions == 1))) {
+        (m->form == Form::kLwe || m->form == Form::kTrlwe)) {
         Candidate c{KernelKind::kTc, kTcSliceWords, 1, kTcMaxK, 0, 0, 1};
         out.push_back(c);
     }

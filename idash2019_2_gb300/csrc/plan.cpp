@@ -312,8 +312,6 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
     *plan = Plan();
     if (in.n_out >= kNoOutput) return "too many outputs";
     if (in.form == Form::kIntPoly) return "the tensor-core plan serves the TRLWE and LWE forms";
-    if (in.form == Form::kTrlwe && in.num_regions != 1)
-        return "the tensor-core plan reads rows unrotated (NUM_REGIONS = 1)";
     const uint64_t n_out = in.n_out;
     Normalised nm;
     {
@@ -365,8 +363,6 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
             win.swap(merged);
             ++e;
         }
-        for (uint64_t k : win)
-            if ((k & 0xFFFFFFFFu) != 0) return "the tensor-core plan reads rows unrotated";
         PlanBlock b{};
         b.slot_begin = uint32_t(plan->slots.size());
         b.n_slots = uint16_t(win.size());
@@ -377,8 +373,8 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         b.term_begin = 0;
         for (size_t c0 = 0, c = 0; c0 < win.size(); c0 += 32, ++c) {
             const size_t c1 = std::min(win.size(), c0 + 32);
-            bool run = true;
-            for (size_t k = c0 + 1; k < c1 && run; ++k) run = (win[k] >> 32) == (win[c0] >> 32) + (k - c0);
+            bool run = uint32_t(win[c0]) == 0;
+            for (size_t k = c0 + 1; k < c1 && run; ++k) run = win[k] == win[c0] + (uint64_t(k - c0) << 32);
             if (run && c < 32) b.term_begin |= 1u << c;
             ++chunks;
             scattered += !run;
@@ -388,7 +384,7 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         b.out_hi = uint32_t(e);
         uint32_t max_row = 0, min_row = win.empty() ? 0u : 0xFFFFFFFFu;
         for (uint64_t k : win) {
-            plan->slots.push_back(PlanSlot{uint32_t(k >> 32), 0});
+            plan->slots.push_back(PlanSlot{uint32_t(k >> 32), uint32_t(k)});
             max_row = std::max(max_row, uint32_t(k >> 32));
             min_row = std::min(min_row, uint32_t(k >> 32));
         }
@@ -418,6 +414,14 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         o = e;
     }
     plan->tc_producers = 4 * scattered > chunks ? kTcMaxProducers : 1;
+    uint32_t rotations = 0;  // all of them, or-ed
+    for (uint64_t k : nm.nkey) rotations |= uint32_t(k);
+    if (rotations) {
+        // a tile of columns is inside one polynomial, and a rotation a mask
+        if (in.N % 64 != 0 || (in.N & (in.N - 1)) != 0) return "the tensor-core plan rotates rows of 2^k >= 64 coefficients";
+        plan->tc_rot_bytes = rotations & 1u ? 4 : rotations & 2u ? 8 : 16;
+        plan->tc_producers = kTcRotProducers;
+    }
     plan->phase_begin.push_back(uint32_t(plan->blocks.size()));
     return "";
 }

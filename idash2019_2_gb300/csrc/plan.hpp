@@ -113,15 +113,16 @@ struct Plan {
     std::vector<uint8_t> tc_a;
     std::vector<TcOut> tc_out;
     uint32_t tc_producers = 1;  // kTcMaxProducers where more than a quarter of the 32-row chunks are scattered rows
+    uint32_t tc_rot_bytes = 0;  // rotated rows: the largest copy (4, 8 or 16 bytes) that every rotation keeps aligned; 0: none
 };
 
 // Tensor-core plans (build_tc_plan).  A block is up to kTcRows consecutive
 // outputs (the MMA's M, one TMEM lane each) over the sorted union of their
-// input rows (the MMA's K, padded to a multiple of 16).  PlanBlock fields are
-// read as: slot_begin/n_slots the rows, n_rot 0, group_begin the offset of the
+// slots, input rows and their rotations (the MMA's K, padded to a multiple of 16).  PlanBlock fields are
+// read as: slot_begin/n_slots the slots, n_rot 0, group_begin the offset of the
 // block's coefficient digits in tc_a in 16-byte units, n_groups the padded K,
-// term_begin a bit mask of the block's 32-row chunks whose rows are
-// consecutive (bit c: rows 32c .. min(32c + 32, n_slots) - 1; such a chunk is
+// term_begin a bit mask of the block's 32-slot chunks whose rows are
+// consecutive and as stored (bit c: rows 32c .. min(32c + 32, n_slots) - 1; such a chunk is
 // one 2D tensor copy), n_terms the block's nonzero terms, out_lo/out_hi its
 // outputs.
 //
@@ -139,6 +140,7 @@ constexpr uint32_t kTcRows = 128;
 // chunk is one tensor copy (5 neighbours, consecutive rows: 0.421 and 0.430).
 constexpr uint32_t kTcMaxProducers = 2;
 constexpr uint32_t kTcMaxK = 192;  // shared-memory bound on the padded K
+constexpr uint32_t kTcRotProducers = 6;  // row-loading warps where rows are rotated (one, two or four words a copy)
 struct TcLimits {
     uint32_t max_k = kTcMaxK;
 };

@@ -72,6 +72,10 @@ struct ScoreArgs {
     uint32_t unit_slices, units_per_block, n_units;
     uint32_t tc_a_max_bytes;      // shared-memory room for one block's digits
     uint32_t tc_producers;        // row-loading warps (Plan::tc_producers)
+    uint32_t tc_rot_bytes;        // rotated slots (Plan::tc_rot_bytes)
+    // with them, n_slices are those with a column that is not zeroed (from N +
+    // region_size on); zero_slices follow them, zero_per_unit for each unit of a block
+    uint32_t zero_slices, zero_per_unit;
     uint32_t unit_step_blocks, unit_step_parts;  // set by the launch: gridDim.x units in blocks and units of a block
     uint32_t tc_use_map, tc_store_map;  // set by the launch: rows come, and outputs go, by tensor copies
     uint32_t tc_a_stages, tc_dig_stages, tc_raw_stages;  // set by the launch: buffers of each kind
@@ -152,7 +156,7 @@ cudaError_t launch_finalize(const FinalizeArgs &a, cudaStream_t stream);
 // Tensor-core kernel (score_tc.cu): dynamic shared memory for a plan whose
 // largest padded K is max_k_pad, its launch (grid = ctas, one per SM at
 // most), and the one-off shared-memory attribute.
-size_t tc_smem_bytes(uint32_t max_k_pad);
+size_t tc_smem_bytes(uint32_t max_k_pad, bool rotated);
 cudaError_t launch_score_tc(const ScoreArgs &a, uint32_t ctas, cudaStream_t stream);
 cudaError_t configure_tc_kernel(size_t max_smem);
 

@@ -47,6 +47,12 @@
 //               and stored by 2D tensor copies of 32 rows x 32 columns, or
 //               row by row where the 32 rows are not all wanted or not
 //               consecutive.
+// Several regions to a row (kRotated): a slot is a row times X^(-m), so the
+// producers (six warps) copy a slot's columns from m on, round the
+// polynomial's end, in the largest pieces that stay aligned, and the
+// converters negate those that went round.  The slices past the last region's
+// columns are zeros: the digits' warp stores them from a box of zeros, and
+// they cost the other roles nothing.
 // What bounds it, and what it measured: 5 neighbours (K = 64, 2.4 GB) the
 // roles' instructions, about 5200 a tile: 0.42 ms against 0.36 ms of memory
 // traffic; 30 neighbours (K = 192) the conversion and the MMAs, 448 cycles of
@@ -75,12 +81,14 @@ constexpr uint32_t kM = kTcRows;        // 128 outputs per block
 constexpr uint32_t kChunk = 32;         // rows per pipeline chunk (two MMA K-steps)
 constexpr uint32_t kMaxChunks = kTcMaxK / kChunk;
 constexpr uint32_t kAccStages = 2;
+constexpr uint32_t kTcRotStages = 6;  // raw stages where rows are rotated
 constexpr uint32_t kMaxAStages = 2, kMaxRawStages = 8, kMaxDigStages = 4;
 constexpr uint32_t kRawStageBytes = kChunk * kN * 4;
 constexpr uint32_t kGroupBytes = 4 * kN * 16;           // 8 rows of the four planes
 constexpr uint32_t kDigStageBytes = (kChunk / 8) * kGroupBytes;
 constexpr uint32_t kOutBox = 32 * 32 * 4;               // one stored box: 32 rows x 32 columns
 constexpr uint32_t kHeader = 2048;
+constexpr uint32_t kZeroBox = 12 * 1024, kRotHeader = kZeroBox + kOutBox;  // with TcRot and a box of zeros
 // Warps: kEpi teams of eight (one, or one per accumulator stage), kProducers
 // producers, one each of MMA and digit loads, then kConv converter teams of
 // kConvWarps.  A parity tells only two successive phases of a barrier apart,
@@ -112,16 +120,24 @@ struct TcShape {
     uint32_t a_stages;    // blocks' coefficient digits
     uint32_t dig_stages;  // chunks of byte planes
     uint32_t raw_stages;  // chunks of ciphertext words
-    constexpr size_t smem(uint32_t k) const {
-        const size_t n = kHeader + a_stages * size_t(tc_a_bytes(k)) + dig_stages * size_t(kDigStageBytes) +
-                         raw_stages * size_t(kRawStageBytes) + kEpiWarps * epi * size_t(kOutBox);
+    constexpr size_t smem(uint32_t k, bool rotated) const {
+        const size_t n = (rotated ? kRotHeader : kHeader) + a_stages * size_t(tc_a_bytes(k)) +
+                         dig_stages * size_t(kDigStageBytes) + raw_stages * size_t(kRawStageBytes) + kEpiWarps * epi * size_t(kOutBox);
         return n < kMinSmem ? kMinSmem : n;
     }
 };
 constexpr TcShape kTcShapes[] = {{2, 2, 2, 2, 2, 8}, {2, 2, 2, 2, 2, 6}, {1, 3, 4, 2, 3, 6}, {1, 3, 4, 1, 3, 6}};
-const TcShape *tc_shape(uint32_t k) {
+// Rotated rows: the producers are most of the work.
+constexpr TcShape kTcRotShapes[] = {{1, 2, 4, 2, 2, 6}, {1, 2, 4, 1, 2, 6}};
+static_assert(kTcShapes[3].smem(kTcMaxK, false) <= kMaxSmem && kTcRotShapes[1].smem(kTcMaxK, true) <= kMaxSmem, "K");
+const TcShape *tc_shape(uint32_t k, bool rotated) {
+    if (rotated) {
+        for (const TcShape &x : kTcRotShapes)
+            if (x.smem(k, true) <= kMaxSmem) return &x;
+        return nullptr;
+    }
     for (const TcShape &x : kTcShapes)
-        if (x.smem(k) <= kMaxSmem) return &x;
+        if (x.smem(k, false) <= kMaxSmem) return &x;
     return nullptr;
 }
 
@@ -135,6 +151,16 @@ struct TcBars {
     uint32_t rows[kTcMaxProducers][kTcMaxK];  // the unit's input rows, per producer
 };
 static_assert(sizeof(TcBars) <= kHeader, "header area");
+
+// Plans with rotated slots: the unit's input rows and rotations, per producer;
+// and per raw stage, slot i's columns from[i] .. 63 are to be negated (they
+// went round the polynomial's end), if any slot's are.
+struct TcRot {
+    uint32_t rows[kTcRotProducers][kTcMaxK], rots[kTcRotProducers][kTcMaxK];
+    uint32_t from[kTcRotStages][kChunk];
+    uint32_t any[kTcRotStages];
+};
+static_assert(kHeader + sizeof(TcRot) <= kZeroBox, "header area");
 
 // A position in a ring of n stages; parity of the round.
 struct Ring {
@@ -225,6 +251,13 @@ struct Units {
     __device__ __forceinline__ uint32_t s1(const ScoreArgs &a) const {
         return min((part + 1) * a.unit_slices, a.n_slices);
     }
+    // the unit's share of the slices that are zeros
+    __device__ __forceinline__ uint32_t z0(const ScoreArgs &a) const {
+        return a.n_slices + min(part * a.zero_per_unit, a.zero_slices);
+    }
+    __device__ __forceinline__ uint32_t z1(const ScoreArgs &a) const {
+        return a.n_slices + min((part + 1) * a.zero_per_unit, a.zero_slices);
+    }
     __device__ __forceinline__ const PlanBlock *header(const ScoreArgs &a) const {
         return a.blocks + a.block_lo + block;
     }
@@ -276,7 +309,49 @@ __device__ __forceinline__ void load_rows(const ScoreArgs &a, const uint32_t *ro
     if (lane == 0) mbar_arrive(full);
 }
 
-template <uint32_t kEpi, uint32_t kConv, uint32_t kConvWarps, uint32_t kProducers>
+template <uint32_t kBytes>
+__device__ __forceinline__ void cp_async_words(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(kBytes) : "memory");
+}
+
+// (8,000 tags, 24,000 targets, 10 regions to a row: 5 neighbours 0.139 ms, 0.294
+// as sums on CUDA cores, 0.091 the memory traffic alone; 20 neighbours 0.183
+// and 1.123 ms.  Two producers, and the zeros staged by the epilogue: 0.243 and
+// 0.334; six: 0.180 and 0.215.  3 regions, copied word by word: 0.191, 0.323.)
+//
+// Columns [c0, c0 + 64) of n rotated slots into a raw stage: column j of a
+// polynomial of slot X^(-m) * row is the row's word (j + m) mod N, negated
+// where j + m >= N (the converters do that).  kBytes divides every rotation.
+// The whole warp calls it.
+template <uint32_t kBytes>
+__device__ __forceinline__ void load_rotated(const ScoreArgs &a, const uint32_t *rows, const uint32_t *rots, uint32_t n,
+                                             uint32_t c0, uint32_t dst, uint32_t lane) {
+    constexpr uint32_t kWords = kBytes / 4, kLanes = kN / kWords;  // lanes of a slot's 64 words
+    const uint32_t mask = a.N - 1, poly = c0 & ~mask, word = lane * kWords % kN;
+    const uint32_t j = (c0 & mask) + word;
+    const uint8_t *base = a.in + uint64_t(poly) * 4;
+    dst += lane * kBytes;  // lanes past a slot's are at the next one's
+    if (kLanes <= 32) {
+        constexpr uint32_t kSlots = kLanes <= 32 ? 32 / kLanes : 1;
+#pragma unroll 4
+        for (uint32_t i = 0; i < n; i += kSlots) {
+            const uint32_t s = min(i + lane / kLanes, n - 1);
+            const uint8_t *src = base + uint64_t(rows[s]) * a.in_stride + ((j + rots[s]) & mask) * 4;
+            cp_async_words<kBytes>(dst + i * (kN * 4), src);
+        }
+    } else {
+#pragma unroll 4
+        for (uint32_t i = 0; i < n; ++i) {
+            const uint8_t *row = base + uint64_t(rows[i]) * a.in_stride;
+            const uint32_t t = j + rots[i];
+            cp_async_words<kBytes>(dst + i * (kN * 4), row + (t & mask) * 4);
+            cp_async_words<kBytes>(dst + i * (kN * 4) + 128, row + ((t + 32) & mask) * 4);
+        }
+    }
+}
+
+// kRotated: rows come rotated (several regions to a row), by kTcRotProducers warps.
+template <uint32_t kEpi, uint32_t kConv, uint32_t kConvWarps, uint32_t kProducers, bool kRotated = false>
 __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers), 1)
     k_score_tc(const __grid_constant__ ScoreArgs a, const __grid_constant__ TcMaps maps) {
     constexpr uint32_t kProducerWarp = kEpiWarps * kEpi, kMmaWarp = kProducerWarp + kProducers;
@@ -284,7 +359,8 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
     constexpr uint32_t kConvWarp0 = kDigitWarp + 1;
     extern __shared__ __align__(1024) uint8_t smem[];
     TcBars &sh = *reinterpret_cast<TcBars *>(smem);
-    uint8_t *stage_out = smem + kHeader;
+    TcRot &rot = *reinterpret_cast<TcRot *>(smem + kHeader);  // kRotated
+    uint8_t *stage_out = smem + (kRotated ? kRotHeader : kHeader);
     uint8_t *smA = stage_out + kEpiWarps * kEpi * kOutBox;
     uint8_t *dig = smA + a.tc_a_stages * a.tc_a_max_bytes;
     uint8_t *raw = dig + a.tc_dig_stages * kDigStageBytes;
@@ -311,6 +387,10 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
         sh.abort = 0;
         fence_mbar_init();
     }
+    if (kRotated && threadIdx.x < kOutBox / 16) {
+        sts_v4(smem_addr(smem + kZeroBox) + threadIdx.x * 16, 0, 0, 0, 0);
+        fence_proxy_async_smem();
+    }
     if (warp == kMmaWarp) tmem_alloc(&sh.tmem_base, kTmemCols);
     tc_fence_before();
     __syncthreads();
@@ -331,7 +411,20 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                 bulk_g2s(smA + ra.s * a.tc_a_max_bytes, src, bytes, &sh.a_full[ra.s]);
                 ++loads;
                 ra.next(a.tc_a_stages);
+                if (kRotated && a.tc_store_map) {
+                    // the unit's share of the slices that are zeros, where whole
+                    // boxes go out (the epilogue stores the others)
+                    const uint32_t z0 = w.z0(a), z1 = w.z1(a), lo = h->out_lo, hi = h->out_hi;
+                    for (uint32_t o = lo; o + 32 <= hi && z0 < z1; o += 32) {
+                        if (o < a.out_lo || uint64_t(o) + 32 > a.out_hi) continue;
+                        for (uint32_t c = z0 * kN; c < z1 * kN; c += 32)
+                            tma_store_2d(&maps.out, int32_t(c), int32_t(o - uint32_t(a.out_row_base)),
+                                         smem_addr(smem + kZeroBox));
+                    }
+                    bulk_commit();
+                }
             }
+            if (kRotated) bulk_wait();
             // let every copy land: the last fill of each buffer (immediate when nothing aborted)
             for (uint32_t k = 1; k <= a.tc_a_stages && k <= loads; ++k) {
                 const uint32_t j = loads - k;
@@ -346,7 +439,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
         // the lookups in it, it took 850 cycles per chunk and bound the kernel.
         struct Rows {
             uint32_t n_slots, runs, n_chunks;  // runs: the block's consecutive-chunk mask
-            uint32_t row[kMaxChunks];          // lane i: row i of each chunk
+            uint32_t row[kMaxChunks], rot[kMaxChunks];  // lane i: slot i of each chunk
         };
         const bool leader = elect_one();
         // Each of the producers takes its chunks in turn (the raw stages are a
@@ -354,7 +447,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
         // second (10 neighbours over permuted rows: one 0.327, two 0.261 ms);
         // boxes are not (headline 0.421 and 0.430 ms).
         const uint32_t me = warp - kProducerWarp;
-        uint32_t *rows = sh.rows[me];
+        uint32_t *rows = kRotated ? rot.rows[me] : sh.rows[me], *rots = rot.rots[me];
         uint32_t turn = 0;
         Units head(a);
         PlanBlock blk{};
@@ -369,7 +462,11 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
             next.n_chunks = (blk.n_groups + kChunk - 1) / kChunk;
 #pragma unroll
             for (uint32_t c = 0; c < kMaxChunks; ++c)
-                if (kChunk * c + lane < blk.n_slots) next.row[c] = a.slots[blk.slot_begin + kChunk * c + lane].row;
+                if (kChunk * c + lane < blk.n_slots) {
+                    const PlanSlot slot = a.slots[blk.slot_begin + kChunk * c + lane];
+                    next.row[c] = slot.row;
+                    if (kRotated) next.rot[c] = slot.rot;
+                }
         };
         fetch_header();
         fetch_rows();
@@ -390,6 +487,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                     r = 0;
                 }
                 rows[kChunk * c + lane] = r;
+                if (kRotated) rots[kChunk * c + lane] = x.rot[c];
             }
             __syncwarp();
             // lane c: the first row of chunk c; the chunks that one tensor copy
@@ -416,13 +514,30 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                         break;
                     if ((boxes >> c) & 1u) {
                         if (leader) {
+                            if (kRotated) rot.any[rr.s] = 0;
                             fence_proxy_async_smem();  // after the converters' reads of the stage
                             mbar_arrive_expect_tx(full, kRawStageBytes);
                             tma_load_2d(dst, &maps.rows, int32_t(c0), r0, full);
                         }
+                    } else if (kRotated && x.n_slots > kChunk * c) {
+                        const uint32_t n = min(kChunk, x.n_slots - kChunk * c);
+                        const uint32_t *r = rows + kChunk * c, *m = rots + kChunk * c;
+                        if (a.tc_rot_bytes == 16) load_rotated<16>(a, r, m, n, c0, smem_addr(dst), lane);
+                        else if (a.tc_rot_bytes == 8) load_rotated<8>(a, r, m, n, c0, smem_addr(dst), lane);
+                        else load_rotated<4>(a, r, m, n, c0, smem_addr(dst), lane);
+                        // columns that stay in the polynomial, from c0 on
+                        const uint32_t to_end = a.N - (c0 & (a.N - 1));
+                        const uint32_t stay = lane < n ? to_end - min(m[lane], to_end) : kN;
+                        rot.from[rr.s][lane] = stay;
+                        const bool any = __any_sync(0xFFFFFFFFu, stay < kN);
+                        if (lane == 0) rot.any[rr.s] = any;
+                        cp_async_arrive(full);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(full);
                     } else if (x.n_slots > kChunk * c) {
                         load_rows(a, rows + kChunk * c, min(kChunk, x.n_slots - kChunk * c), c0, smem_addr(dst), full, lane);
                     } else if (leader) {
+                        if (kRotated) rot.any[rr.s] = 0;
                         mbar_arrive(full);  // rows of padding only: their coefficients are zero
                     }
                     __syncwarp();
@@ -472,6 +587,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                     // are here.  Volatile loads: with plain ones the compiler
                     // moved them below the arrival and the wait that follow.
                     uint32_t w[kUnits][8];
+                    const bool negate = kRotated && *reinterpret_cast<volatile uint32_t *>(&rot.any[rr.s]) != 0;
 #pragma unroll
                     for (uint32_t x = 0; x < kUnits; ++x) {
                         const uint32_t q = x * kTeamThreads + tid, g = q / kN, col = q % kN;
@@ -482,6 +598,14 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                                          : "=r"(w[x][r])
                                          : "r"(src + ((8 * g + r) * kN + col) * 4)
                                          : "memory");
+                        if (negate) {
+                            const uint32_t at = smem_addr(&rot.from[rr.s][8 * g]);
+                            const uint4 f0 = lds_v4_ordered(at), f1 = lds_v4_ordered(at + 16);
+                            const uint32_t from[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+#pragma unroll
+                            for (uint32_t r = 0; r < 8; ++r)
+                                if (col >= from[r]) w[x][r] = 0u - w[x][r];
+                        }
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sh.raw_empty[rr.s]);
@@ -701,6 +825,18 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                 }
                 __syncwarp();  // the warp has read its staged rows before they are overwritten
             }
+            if (!kRotated) continue;
+            // the unit's share of the slices that are zeros; the teams in turn
+            const uint32_t z0 = w.z0(a), z1 = w.z1(a);
+            if (!ok || boxes || z0 + team >= z1) continue;
+            for (uint32_t i = 0; i < 8; ++i) {
+                const uint64_t dst = __shfl_sync(0xFFFFFFFFu, reinterpret_cast<uint64_t>(orow), 4 * i + lane / 8);
+                if (!dst) continue;
+                for (uint32_t sl = z0 + team; sl < z1; sl += kEpi) {
+                    const uint32_t c = sl * kN + 32 * half + 4 * (lane % 8);
+                    for (uint32_t e = c; e < min(c + 4, a.row_words); ++e) reinterpret_cast<uint32_t *>(dst)[e] = 0u;
+                }
+            }
         }
         if (lane == 0) bulk_wait();  // the stored boxes are written
     }
@@ -744,13 +880,14 @@ bool encode_rows_map(const uint8_t *base, uint64_t words, uint64_t rows, uint64_
 
 }  // namespace
 
-size_t tc_smem_bytes(uint32_t max_k_pad) {
-    const TcShape *x = tc_shape(max_k_pad);
-    return x ? x->smem(max_k_pad) : SIZE_MAX;
+size_t tc_smem_bytes(uint32_t max_k_pad, bool rotated) {
+    const TcShape *x = tc_shape(max_k_pad, rotated);
+    return x ? x->smem(max_k_pad, rotated) : SIZE_MAX;
 }
 
 cudaError_t configure_tc_kernel(size_t max_smem) {
-    for (auto *fn : {k_score_tc<2, 2, 2, 1>, k_score_tc<2, 2, 2, 2>, k_score_tc<1, 3, 4, 1>, k_score_tc<1, 3, 4, 2>}) {
+    for (auto *fn : {k_score_tc<2, 2, 2, 1>, k_score_tc<2, 2, 2, 2>, k_score_tc<1, 3, 4, 1>, k_score_tc<1, 3, 4, 2>,
+                     k_score_tc<1, 2, 4, kTcRotProducers, true>}) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(max_smem));
         if (e != cudaSuccess) return e;
     }
@@ -763,12 +900,14 @@ cudaError_t launch_score_tc(const ScoreArgs &a_in, uint32_t ctas, cudaStream_t s
         return cudaErrorInvalidValue;
     ScoreArgs a = a_in;
     const uint32_t k = a.tc_a_max_bytes / uint32_t(tc_a_bytes(1));
-    const TcShape *shape = tc_shape(k);
+    const bool rotated = a.tc_rot_bytes != 0;
+    const TcShape *shape = tc_shape(k, rotated);
     if (!shape) return cudaErrorInvalidValue;
     a.tc_a_stages = shape->a_stages;
     a.tc_dig_stages = shape->dig_stages;
     a.tc_raw_stages = shape->raw_stages;
-    if (a.tc_producers == 0 || a.tc_producers > kTcMaxProducers) return cudaErrorInvalidValue;
+    if (a.tc_producers == 0 || (rotated ? a.tc_producers != kTcRotProducers : a.tc_producers > kTcMaxProducers))
+        return cudaErrorInvalidValue;
     TcMaps maps;
     std::memset(&maps, 0, sizeof(maps));
     a.tc_use_map = encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, kChunk, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -780,9 +919,11 @@ cudaError_t launch_score_tc(const ScoreArgs &a_in, uint32_t ctas, cudaStream_t s
     a.unit_step_blocks = grid / a.units_per_block;
     a.unit_step_parts = grid % a.units_per_block;
     const bool two = a.tc_producers == 2;
-    auto *fn = shape->epi == 2 ? (two ? k_score_tc<2, 2, 2, 2> : k_score_tc<2, 2, 2, 1>)
+    auto *fn = rotated           ? k_score_tc<1, 2, 4, kTcRotProducers, true>
+               : shape->epi == 2 ? (two ? k_score_tc<2, 2, 2, 2> : k_score_tc<2, 2, 2, 1>)
                                : (two ? k_score_tc<1, 3, 4, 2> : k_score_tc<1, 3, 4, 1>);
-    fn<<<grid, tc_threads(shape->epi, shape->conv, shape->conv_warps, a.tc_producers), shape->smem(k), stream>>>(a, maps);
+    const uint32_t threads = tc_threads(shape->epi, shape->conv, shape->conv_warps, a.tc_producers);
+    fn<<<grid, threads, shape->smem(k, rotated), stream>>>(a, maps);
     return cudaGetLastError();
 }
 

@@ -94,3 +94,48 @@ def test_lwe(ctx, oracle, n, n_indiv, k, scatter):
     m.free()
     d_in.free()
     d_out.free()
+
+
+@pytest.mark.parametrize("regions,size,ns", [
+    (1, 800, 799), (2, 512, 512), (3, 341, 300), (3, 340, 1), (7, 146, 100), (10, 102, 101), (16, 64, 64), (40, 25, 25),
+    (341, 3, 2), (1024, 1, 1)])
+@pytest.mark.parametrize("tags,targets,neighbours", [(60, 90, 1), (130, 100, 5), (100, 45, 25)])
+def test_rotated_rows(ctx, oracle, regions, size, ns, tags, targets, neighbours):
+    """Several regions to a row: rotations that keep 16, 8 and 4 bytes aligned,
+    tiles before, at and after a polynomial's end, and columns that are zeros;
+    dense outputs, a range of them, and records through a row map."""
+    w = gpu.synth_model(seed=regions + neighbours, n_tags=tags, n_targets=targets, neighbours=neighbours)
+    csr, n_rows = w.model, (3 * tags + regions - 1) // regions
+    rng = np.random.default_rng(regions)
+    rows = _words(rng, (n_rows, 2048))
+    rows[0, ::3] = -2 ** 31
+    want, _ = oracle.trlwe_score(csr.term_ptr, csr.term_feat, csr.term_coef, rows, ns, regions, size)
+    m = gpu.TrlweModel(ctx, csr, n_rows, ns, regions, size)
+    assert m.info()["kernel"] == TC_KIND
+    d_in, d_out = ctx.device_alloc(rows.nbytes), ctx.device_alloc(m.n_out * gpu.RECORD_BYTES + 16)
+    d_in.upload(rows)
+    for graph in (1, 0):
+        ctx.set_option("graph", graph)
+        d_out.upload(np.full(m.n_out * 2048, 77, np.int32))
+        m.score_device(d_in.ptr, gpu.DENSE_TRLWE, d_out.ptr, gpu.DENSE_TRLWE)
+        ctx.sync()
+        got = d_out.download(nbytes=m.n_out * 8192, dtype=np.int32).reshape(m.n_out, 2048)
+        np.testing.assert_array_equal(got, want)
+    ctx.set_option("graph", 1)
+    lo, hi = 2, m.n_out - 3
+    d_out.upload(np.full(m.n_out * 2048, 77, np.int32))
+    m.score_range(lo, hi, 0, d_in.ptr, gpu.DENSE_TRLWE, 0, n_rows, d_out.ptr, gpu.DENSE_TRLWE)
+    ctx.sync()
+    got = d_out.download(nbytes=m.n_out * 8192, dtype=np.int32).reshape(m.n_out, 2048)
+    np.testing.assert_array_equal(got[:hi - lo], want[lo:hi])
+    assert (got[hi - lo:] == 77).all()
+    m.free()
+    out_row = rng.permutation(csr.n_out).astype(np.uint32)
+    m = gpu.TrlweModel(ctx, csr, n_rows, ns, regions, size, out_row=out_row)
+    m.score_device(d_in.ptr, gpu.DENSE_TRLWE, d_out.ptr + 8, gpu.RECORD_OUT)
+    ctx.sync()
+    got = d_out.download(nbytes=m.n_out * gpu.RECORD_BYTES, offset=8, dtype=np.int32).reshape(m.n_out, -1)
+    np.testing.assert_array_equal(got[out_row, 2:2050], want)
+    m.free()
+    d_in.free()
+    d_out.free()
