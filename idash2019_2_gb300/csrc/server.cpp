@@ -23,10 +23,16 @@
 //               segments), and the rest follows at once behind it: the
 //               device then always has a launch queued while the requests
 //               of the one before complete and new ones are staged;
-//   completion  a launched segment's outputs go back to host memory on the
-//               output stream (when the request has a host buffer), its
-//               segment memory returns to the arena; when every segment of a
-//               request is back, its digest is read and it completes.
+//   outputs     a launch's outputs go back to page-locked host memory on the
+//               output stream, and the digest of each request whose last
+//               segment it holds: all queued behind the launch when it is
+//               issued, so that the host is in no step between scoring and
+//               completion (it was in three: one request of 10 targets took
+//               281 us, now 115; nine of 6 targets 491, now 266).  Copies to
+//               pageable memory would hold the thread up until the launch is
+//               done, so those are issued after it, on a stream of their own;
+//   completion  a copied segment's memory returns to the arena; a request
+//               completes when its digest is here.
 // The digest of a request is taken by the scoring kernel as it stores the
 // outputs, per job, into the request's own digest slot: it depends only on the
 // request's own outputs, not on what shared the launch.
@@ -40,6 +46,8 @@
 #include <mutex>
 #include <thread>
 #include <vector>
+
+#include <sys/prctl.h>
 
 #include "capi_internal.hpp"
 
@@ -122,6 +130,7 @@ struct Req {
     size_t next_seg = 0, segs_done = 0;
     uint32_t digest_slot = 0;
     cudaEvent_t finished = nullptr;
+    bool pageable = false;  // h_out is not page-locked
     ReqState state = ReqState::kQueued;
     idash_status status = IDASH_PENDING;
     idash_request_result res{};
@@ -143,7 +152,7 @@ struct idash_server {
     std::vector<uint32_t> free_slots;
     uint32_t *d_counters = nullptr;
     uint32_t next_counter = 0;
-    cudaStream_t compute = nullptr, h2d = nullptr, d2h = nullptr;
+    cudaStream_t compute = nullptr, h2d = nullptr, d2h = nullptr, late = nullptr;  // late: copies to pageable memory
     cudaEvent_t t0 = nullptr;
     ScoreJob *d_jobs[kLaunchRing] = {};
     ScoreJob *h_jobs[kLaunchRing] = {};
@@ -196,6 +205,8 @@ struct idash_server {
     bool stage(Req *q, Segment &g);
     bool stage_segments();
     bool launch();
+    bool copy_outputs(Req *q, Segment &g, cudaStream_t s);
+    bool finish(Req *q, cudaStream_t s);
     bool complete();
     void run();
 };
@@ -276,6 +287,11 @@ bool idash_server::admit(Req *q) {
     q->next_seg = 1;
     q->digest_slot = free_slots.back();
     free_slots.pop_back();
+    if (q->r.h_out) {
+        cudaPointerAttributes at{};
+        q->pageable = cudaPointerGetAttributes(&at, q->r.h_out) != cudaSuccess || at.type != cudaMemoryTypeHost;
+        if (q->pageable) cudaGetLastError();
+    }
     q->res.admit_s = now_s();
     q->res.device_bytes = Arena::round(q->segs[0].in_bytes) + Arena::round(q->segs[0].bytes);
     q->state = ReqState::kAdmitted;
@@ -332,7 +348,6 @@ bool idash_server::launch() {
         picks.resize(n);
     }
     std::vector<ScoreJob> jobs;
-    std::vector<Segment *> segs;
     uint64_t tiles = 0;
     for (const Pick &p : picks) {
         {
@@ -364,7 +379,6 @@ bool idash_server::launch() {
                 tiles += uint64_t(j.n_blocks) * n_slices;
                 jobs.push_back(j);
             }
-            segs.push_back(&g);
         }
     }
     if (tiles >= 0xFFFFFFFFull) return fail("one launch would exceed 2^32 tiles; lower segment_outputs");
@@ -411,10 +425,16 @@ bool idash_server::launch() {
     if (!check(cudaEventRecord(launch_start[k], compute), "event")) return false;
     if (!check(launch_score(KernelKind::kWs, W, m->group_size, a, m->ctas, compute), "scoring launch")) return false;
     if (!check(cudaEventRecord(launch_done[k], compute), "event")) return false;
-    for (Segment *g : segs) {
-        g->state = SegState::kLaunched;
-        g->launch = k;
-        g->launch_seq = launch_seq;
+    if (!check(cudaStreamWaitEvent(d2h, launch_done[k], 0), "wait for a launch")) return false;
+    for (const Pick &p : picks) {
+        p.g->state = SegState::kLaunched;
+        p.g->launch = k;
+        p.g->launch_seq = launch_seq;
+        if (p.q->pageable) continue;
+        if (p.q->r.h_out && !copy_outputs(p.q, *p.g, d2h)) return false;
+        bool last = p.q->next_seg == p.q->segs.size();
+        for (const Segment &g : p.q->segs) last = last && g.state != SegState::kWaiting && g.state != SegState::kStaged;
+        if (last && !finish(p.q, d2h)) return false;
     }
     ++launch_seq;
     launches.fetch_add(1);
@@ -423,6 +443,34 @@ bool idash_server::launch() {
         ++stats.launches;
     }
     return true;
+}
+
+// Queues the copies of segment g's outputs to the request's host buffer.
+bool idash_server::copy_outputs(Req *q, Segment &g, cudaStream_t s) {
+    const uint64_t n_req = q->out_end - q->out_begin, n_seg = g.o_hi - g.o_lo;
+    for (uint32_t b = 0; b < q->blocks; ++b) {
+        uint8_t *dst =
+            static_cast<uint8_t *>(q->r.h_out) + (uint64_t(b) * n_req + (g.o_lo - q->out_begin)) * q->row_bytes;
+        if (!check(cudaMemcpyAsync(dst, arena_base + g.off + uint64_t(b) * n_seg * q->row_bytes, n_seg * q->row_bytes,
+                                   cudaMemcpyDeviceToHost, s),
+                   "request outputs"))
+            return false;
+    }
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        stats.d2h_bytes += q->blocks * n_seg * q->row_bytes;
+    }
+    g.copied = take_event();
+    return check(cudaEventRecord(g.copied, s), "event");
+}
+
+// Queues the read of the request's digest, after its last segment.
+bool idash_server::finish(Req *q, cudaStream_t s) {
+    if (!check(cudaMemcpyAsync(h_digest + q->digest_slot, d_digest + q->digest_slot, 8, cudaMemcpyDeviceToHost, s),
+               "digest"))
+        return false;
+    q->finished = take_event();
+    return check(cudaEventRecord(q->finished, s), "event");
 }
 
 bool idash_server::complete() {
@@ -445,21 +493,7 @@ bool idash_server::complete() {
         for (Segment &g : q->segs) {
             if (g.state == SegState::kLaunched && g.launch_seq < launch_retired) {
                 if (q->r.h_out) {
-                    const uint64_t n_req = q->out_end - q->out_begin, n_seg = g.o_hi - g.o_lo;
-                    for (uint32_t b = 0; b < q->blocks; ++b) {
-                        uint8_t *dst = static_cast<uint8_t *>(q->r.h_out) +
-                                       (uint64_t(b) * n_req + (g.o_lo - q->out_begin)) * q->row_bytes;
-                        if (!check(cudaMemcpyAsync(dst, arena_base + g.off + uint64_t(b) * n_seg * q->row_bytes,
-                                                   n_seg * q->row_bytes, cudaMemcpyDeviceToHost, d2h),
-                                   "request outputs"))
-                            return false;
-                    }
-                    {
-                        std::lock_guard<std::mutex> lock(mu);
-                        stats.d2h_bytes += q->blocks * n_seg * q->row_bytes;
-                    }
-                    g.copied = take_event();
-                    if (!check(cudaEventRecord(g.copied, d2h), "event")) return false;
+                    if (q->pageable && !copy_outputs(q, g, late)) return false;
                     g.state = SegState::kCopying;
                 } else {
                     g.state = SegState::kDone;
@@ -482,13 +516,7 @@ bool idash_server::complete() {
             }
         }
         if (q->state == ReqState::kAdmitted && q->segs_done == q->segs.size()) {
-            // every launch of this request is complete: read its digest
-            if (!check(cudaMemcpyAsync(h_digest + q->digest_slot, d_digest + q->digest_slot, 8,
-                                       cudaMemcpyDeviceToHost, d2h),
-                       "digest"))
-                return false;
-            q->finished = take_event();
-            if (!check(cudaEventRecord(q->finished, d2h), "event")) return false;
+            if (q->pageable && !finish(q, late)) return false;
             q->state = ReqState::kFinishing;
         }
         if (q->state == ReqState::kFinishing) {
@@ -519,6 +547,8 @@ bool idash_server::complete() {
 
 void idash_server::run() {
     cudaSetDevice(ctx->device);
+    // the waits of 20 us below are to end after 20 us, not 50 later
+    prctl(PR_SET_TIMERSLACK, 1000UL, 0UL, 0UL, 0UL);
     bool ok = true;
     while (ok) {
         bool idle = true;
@@ -557,6 +587,7 @@ void idash_server::run() {
         cudaStreamSynchronize(compute);
         cudaStreamSynchronize(h2d);
         cudaStreamSynchronize(d2h);
+        cudaStreamSynchronize(late);
         std::lock_guard<std::mutex> lock(mu);
         for (auto &kv : all)
             if (kv.second->state != ReqState::kDone) {
@@ -613,7 +644,7 @@ idash_status idash_server_open(idash_model *m, const idash_serve_config *cfg, id
     for (uint32_t i = 0; i < slots; ++i) s->free_slots.push_back(uint32_t(slots - 1 - i));
     if ((st = ctx->check_cuda(cudaMalloc(&s->d_counters, kCounters * 4), "cudaMalloc(counters)")) != IDASH_OK)
         return bad(st);
-    for (cudaStream_t *x : {&s->compute, &s->h2d, &s->d2h})
+    for (cudaStream_t *x : {&s->compute, &s->h2d, &s->d2h, &s->late})
         if ((st = ctx->check_cuda(cudaStreamCreateWithFlags(x, cudaStreamNonBlocking), "cudaStreamCreate")) != IDASH_OK)
             return bad(st);
     for (uint32_t i = 0; i < kLaunchRing; ++i)
@@ -709,7 +740,7 @@ idash_status idash_server_close(idash_server *s) {
     if (s->worker.joinable()) s->worker.join();
     idash_status st = IDASH_OK;
     if (!s->error.empty()) st = s->ctx->fail(IDASH_ERR_CUDA, s->error);
-    for (cudaStream_t x : {s->compute, s->h2d, s->d2h})
+    for (cudaStream_t x : {s->compute, s->h2d, s->d2h, s->late})
         if (x) cudaStreamSynchronize(x);
     if (st == IDASH_OK) st = idash_sync(s->ctx);
     for (auto &kv : s->all) {
@@ -728,7 +759,7 @@ idash_status idash_server_close(idash_server *s) {
         cudaFreeHost(s->h_jobs[i]);
     }
     if (s->t0) cudaEventDestroy(s->t0);
-    for (cudaStream_t x : {s->compute, s->h2d, s->d2h})
+    for (cudaStream_t x : {s->compute, s->h2d, s->d2h, s->late})
         if (x) cudaStreamDestroy(x);
     cudaFree(s->d_counters);
     cudaFree(s->d_digest);
