@@ -1,6 +1,7 @@
 // C ABI (include/idash_gpu.h): contexts, resident models, the autotuner,
 // CUDA-graph replay and the pipelined host-memory path.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <thread>
@@ -179,6 +180,42 @@ idash_status upload_plan(idash_model *m, const Candidate &c, BuiltPlan &&b) {
 idash_status build_and_upload(idash_model *m, const Candidate &c) { return upload_plan(m, c, make_plan(m, c)); }
 
 
+// Cuts the blocks' column slices into units for `ctas` CTAs that take them in
+// turn.  TRLWE rows as stored: for each number n of units a CTA may get, the
+// largest units that come to no more; then the n where the longest CTA has
+// least to do.  A unit costs half a slice more than it has (its digits and
+// lookups); and where a block is not spread over all CTAs, the longest of some
+// 150 sums of n units of unlike blocks is about 2.5 standard deviations above
+// the mean.  Otherwise about 32 units a CTA: larger ones lose to memory what
+// they save (LWE rows are long, and the units in progress then write few
+// neighbouring columns of many rows: 37 individuals, n = 630, 0.240 ms with 6
+// slices a unit, 0.276 with 22; rows of several regions bring their zeros in
+// bursts: 0.182 and 0.203).  By count and by this rule, 1,000 individuals
+// unless stated: headline 0.420 and 0.413 ms; 3,000 targets, 10 neighbours
+// 51.4 and 47.2 us; 200 targets, 20 neighbours 14.5 and 12.6; 8,000 targets,
+// 700 individuals 60.5 and 51.4.
+void tc_units(ScoreArgs *a, uint32_t ctas, double spread) {
+    const uint64_t blocks = std::max<uint32_t>(a->n_blocks, 1), slices = std::max<uint32_t>(a->n_slices, 1);
+    if (a->form != kFormTrlwe || a->tc_rot_bytes) {
+        const uint64_t want = std::max<uint64_t>(1, uint64_t(ctas) * 32);
+        a->unit_slices = uint32_t(std::min(slices, std::max<uint64_t>(1, (blocks * slices + want - 1) / want)));
+        a->units_per_block = uint32_t((slices + a->unit_slices - 1) / a->unit_slices);
+        a->unit_slices = uint32_t((slices + a->units_per_block - 1) / a->units_per_block);  // evenly
+        return;
+    }
+    const uint64_t least = (blocks + ctas - 1) / ctas;  // a unit per block
+    double best = -1;
+    for (uint64_t n = least; n < least + 48; ++n) {
+        const uint64_t parts = std::min(slices, n * ctas / blocks), unit = (slices + parts - 1) / parts;
+        double cost = double(n) * (double(unit) + 0.5);
+        if (parts < ctas) cost += 2.5 * spread * double(unit) * std::sqrt(double(n));
+        if (best >= 0 && cost >= best) continue;
+        best = cost;
+        a->unit_slices = uint32_t(unit);
+    }
+    a->units_per_block = uint32_t((slices + a->unit_slices - 1) / a->unit_slices);
+}
+
 ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_stride, uint8_t *out_payload,
                     uint64_t out_stride, uint32_t row_words, uint32_t b_lo, uint32_t b_hi, uint64_t out_lo,
                     uint64_t out_hi, uint64_t out_row_base) {
@@ -213,9 +250,8 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
     a.tile_counter = m->ctx->counter();
     a.err = m->ctx->d_err;
     if (m->kind == KernelKind::kTc) {
-        // work units of whole column-slice runs of one block, about 32 per
-        // CTA so the persistent grid balances; the block's coefficient digits
-        // are loaded once per unit
+        // work units of whole column-slice runs of one block, whose
+        // coefficient digits are loaded once per unit
         a.tc_a = m->d_tc_a;
         a.tc_out = m->d_tc_out;
         a.tc_producers = m->plan.tc_producers;
@@ -226,11 +262,7 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
             a.n_slices -= a.zero_slices;
         }
         a.tc_a_max_bytes = uint32_t(tc_a_bytes(m->max_terms));
-        const uint64_t tiles = uint64_t(a.n_blocks) * a.n_slices;
-        const uint64_t want = std::max<uint64_t>(1, uint64_t(m->ctas) * 32);
-        a.unit_slices = uint32_t(std::min<uint64_t>(a.n_slices, std::max<uint64_t>(1, (tiles + want - 1) / want)));
-        a.units_per_block = (a.n_slices + a.unit_slices - 1) / a.unit_slices;
-        a.unit_slices = (a.n_slices + a.units_per_block - 1) / a.units_per_block;  // evenly
+        tc_units(&a, m->ctas, m->plan.tc_spread);
         a.n_units = a.n_blocks * a.units_per_block;
         a.zero_per_unit = (a.zero_slices + a.units_per_block - 1) / a.units_per_block;
     }

@@ -2,6 +2,7 @@
 #include "plan.hpp"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 namespace idash {
@@ -422,6 +423,14 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         plan->tc_rot_bytes = rotations & 1u ? 4 : rotations & 2u ? 8 : 16;
         plan->tc_producers = kTcRotProducers;
     }
+    // a slice of K rows costs about K + 60 (the epilogue)
+    double sum = 0, squares = 0;
+    for (const PlanBlock &b : plan->blocks) {
+        sum += b.n_groups + 60.0;
+        squares += (b.n_groups + 60.0) * (b.n_groups + 60.0);
+    }
+    const double n = double(plan->blocks.size());
+    if (sum > 0) plan->tc_spread = std::sqrt(std::max(0.0, squares * n / (sum * sum) - 1.0));
     plan->phase_begin.push_back(uint32_t(plan->blocks.size()));
     return "";
 }

@@ -113,6 +113,7 @@ struct Plan {
     std::vector<uint8_t> tc_a;
     std::vector<TcOut> tc_out;
     uint32_t tc_producers = 1;  // kTcMaxProducers where more than a quarter of the 32-row chunks are scattered rows
+    double tc_spread = 0;       // standard deviation of a slice's cost over the blocks, in mean costs
     uint32_t tc_rot_bytes = 0;  // rotated rows: the largest copy (4, 8 or 16 bytes) that every rotation keeps aligned; 0: none
 };
 
