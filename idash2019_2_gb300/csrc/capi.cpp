@@ -467,33 +467,63 @@ template <typename TimeFn>
 idash_status autotune(idash_model *m, TimeFn time_fn) {
     const std::vector<Candidate> cands = candidates(m);
     float best = -1.f;
+    bool best_is_current = false;
     Candidate best_c{};
     BuiltPlan best_plan;
+    auto try_plan = [&](const Candidate &c, BuiltPlan &&b) {
+        best_is_current = false;
+        if (upload_plan(m, c, std::move(b)) != IDASH_OK) return;
+        const float ms = time_fn();
+        if (ms > 0 && (best < 0 || ms < best)) {
+            best = ms;
+            best_is_current = true;
+            best_c = c;
+            best_plan.plan = std::move(m->plan);  // given back below, or the next upload replaces it
+        }
+    };
+    // The tensor-core plan is the largest to upload and often the fastest: it
+    // is built with the first ones and timed last of the whole candidates, as
+    // what was timed last needs no second upload when it wins.
+    Candidate late_c{};
+    BuiltPlan late;
+    bool have_late = false;
+    auto try_late = [&]() {
+        if (have_late) try_plan(late_c, std::move(late));
+        have_late = false;
+    };
     bool stop = false;
     const size_t width = std::max<size_t>(1, std::min<size_t>(kPlanThreads, std::thread::hardware_concurrency()));
     for (size_t i = 0; i < cands.size() && !stop; i += width) {
         const size_t n = std::min(width, cands.size() - i);
+        // split candidates are seldom wanted: not built where a whole one is there
+        if (cands[i].split) {
+            try_late();
+            if (best >= 0) break;
+        }
         std::vector<BuiltPlan> built(n);
         std::vector<std::thread> threads;
         for (size_t k = 0; k < n; ++k)
             threads.emplace_back([&, k] { built[k] = make_plan(m, cands[i + k]); });
         for (auto &t : threads) t.join();
-        for (size_t k = 0; k < n; ++k) {
+        for (size_t k = 0; k < n && !stop; ++k) {
             const Candidate &c = cands[i + k];
-            if (c.split && best >= 0) {
-                stop = true;
-                break;
+            if (c.kind == KernelKind::kTc) {
+                late_c = c;
+                late = std::move(built[k]);
+                have_late = true;
+                continue;
             }
-            if (upload_plan(m, c, std::move(built[k])) != IDASH_OK) continue;
-            const float ms = time_fn();
-            if (ms > 0 && (best < 0 || ms < best)) {
-                best = ms;
-                best_c = c;
-                best_plan.plan = std::move(m->plan);  // the next upload replaces the model's plan anyway
+            if (c.split) {
+                try_late();
+                stop = best >= 0;
             }
+            if (!stop) try_plan(c, std::move(built[k]));
         }
     }
-    idash_status s = best < 0 ? plan_default(m) : upload_plan(m, best_c, std::move(best_plan));
+    try_late();
+    idash_status s = IDASH_OK;
+    if (best_is_current) m->plan = std::move(best_plan.plan);
+    else s = best < 0 ? plan_default(m) : upload_plan(m, best_c, std::move(best_plan));
     if (s == IDASH_OK) m->tuned = true;
     return s;
 }
