@@ -54,7 +54,7 @@
 // columns are zeros: the digits' warp stores them from a box of zeros, and
 // they cost the other roles nothing.
 // What bounds it, and what it measured: 5 neighbours (K = 64, 2.4 GB) the
-// roles' instructions, about 5200 a tile: 0.42 ms against 0.36 ms of memory
+// roles' instructions, about 5200 a tile: 0.41 ms against 0.36 ms of memory
 // traffic; 30 neighbours (K = 192) the conversion and the MMAs, 448 cycles of
 // MMA per 32 rows.
 // Every wait is bounded; a wait that expires records IDASH_ERR_DEVICE_TIMEOUT,

@@ -72,7 +72,8 @@ idash_status idash_sync(idash_ctx *ctx);
 
 /* Tunables: "kernel" (0 batched: autotuned among the persistent kernels,
  * 1 plain per-output kernel, 2 single-buffer persistent only, 3 double-buffer
- * persistent only, 4 warp-specialised producer/consumer ring only),
+ * persistent only, 4 warp-specialised producer/consumer ring only, 5 tensor
+ * cores only),
  * "slice_words" (0 = autotune; 128..2048), "ctas_per_sm",
  * "graph" (0/1: replay launches from a CUDA graph), "max_window_slots",
  * "max_group_terms", "split" (1, the default: the batched kernels take
@@ -455,7 +456,8 @@ idash_status idash_encrypt_files(int device, const char *keys_file, const char *
  * d_out[r * num_samples + j] = float(phase_r[j] / 2^32).  key: the key's N
  * integer coefficients in host memory (binary for TFHE keys; any integers
  * are accepted).  N a power of two in [4, 2048].  Asynchronous on `stream`
- * once the key has been staged (the call synchronises with `stream` first). */
+ * once the key has been read: binary keys with N >= 64 travel in the launch
+ * parameters, others are staged in device memory in stream order. */
 idash_status idash_decrypt_trlwe_device(idash_ctx *ctx, const int32_t *key, uint32_t N, const void *d_in,
                                         const idash_row_layout *in_layout, uint64_t n_rows, uint32_t num_samples,
                                         float *d_out, void *stream);
