@@ -181,29 +181,35 @@ idash_status build_and_upload(idash_model *m, const Candidate &c) { return uploa
 
 
 // Cuts the blocks' column slices into units for `ctas` CTAs that take them in
-// turn.  TRLWE rows as stored: for each number n of units a CTA may get, the
-// largest units that come to no more; then the n where the longest CTA has
-// least to do.  A unit costs half a slice more than it has (its digits and
-// lookups); and where a block is not spread over all CTAs, the longest of some
-// 150 sums of n units of unlike blocks is about 2.5 standard deviations above
-// the mean.  Otherwise about 32 units a CTA: larger ones lose to memory what
-// they save (LWE rows are long, and the units in progress then write few
-// neighbouring columns of many rows: 37 individuals, n = 630, 0.240 ms with 6
-// slices a unit, 0.276 with 22; rows of several regions bring their zeros in
-// bursts: 0.182 and 0.203).  By count and by this rule, 1,000 individuals
-// unless stated: headline 0.420 and 0.413 ms; 3,000 targets, 10 neighbours
-// 51.4 and 47.2 us; 200 targets, 20 neighbours 14.5 and 12.6; 8,000 targets,
-// 700 individuals 60.5 and 51.4.
-void tc_units(ScoreArgs *a, uint32_t ctas, double spread) {
+// turn: for each number n of units a CTA may get, the largest units that come
+// to no more; then the n where the longest CTA has least to do.  A unit costs
+// half a slice more than it has (its digits and lookups); and where a block is
+// not spread over all CTAs, the longest of some 150 sums of n units of unlike
+// blocks is about 2.5 standard deviations above the mean.  Against about 32
+// units a CTA, 1,000 individuals unless stated: headline 0.420 and 0.413 ms;
+// 3,000 targets, 10 neighbours 51.4 and 47.2 us; 200 targets, 20 neighbours
+// 14.5 and 12.6; 8,000 targets, 700 individuals 60.5 and 51.4.
+//
+// LWE rows are long: larger units write few neighbouring columns of many rows
+// at a time, and lose to memory what they save (37 individuals, n = 630: 0.240
+// ms with 6 slices a unit, 0.253 with 8, 0.277 with 16, 0.271 with 2; 100
+// individuals, 6,000 outputs: 0.632, 0.648, 0.659 and 0.685), so at most 6.
+// About 32 units a CTA where the digits are not loaded ahead (their load is
+// then worth more slices: 5 to 50 neighbours 5.98 ms, 6.07 with 6 slices) and
+// for rows of several regions (their zeros come in bursts: 0.182 and 0.203).
+void tc_units(ScoreArgs *a, uint32_t ctas, double spread, bool digits_ahead) {
+    constexpr uint64_t kLweUnit = 6;
     const uint64_t blocks = std::max<uint32_t>(a->n_blocks, 1), slices = std::max<uint32_t>(a->n_slices, 1);
-    if (a->form != kFormTrlwe || a->tc_rot_bytes) {
+    const bool lwe = a->form != kFormTrlwe;
+    if (a->tc_rot_bytes || (lwe && !digits_ahead)) {
         const uint64_t want = std::max<uint64_t>(1, uint64_t(ctas) * 32);
         a->unit_slices = uint32_t(std::min(slices, std::max<uint64_t>(1, (blocks * slices + want - 1) / want)));
         a->units_per_block = uint32_t((slices + a->unit_slices - 1) / a->unit_slices);
         a->unit_slices = uint32_t((slices + a->units_per_block - 1) / a->units_per_block);  // evenly
         return;
     }
-    const uint64_t least = (blocks + ctas - 1) / ctas;  // a unit per block
+    const uint64_t least_parts = lwe ? (slices + kLweUnit - 1) / kLweUnit : 1;
+    const uint64_t least = (blocks * least_parts + ctas - 1) / ctas;
     double best = -1;
     for (uint64_t n = least; n < least + 48; ++n) {
         const uint64_t parts = std::min(slices, n * ctas / blocks), unit = (slices + parts - 1) / parts;
@@ -262,7 +268,7 @@ ScoreArgs make_args(idash_model *m, const uint8_t *in_payload, uint64_t in_strid
             a.n_slices -= a.zero_slices;
         }
         a.tc_a_max_bytes = uint32_t(tc_a_bytes(m->max_terms));
-        tc_units(&a, m->ctas, m->plan.tc_spread);
+        tc_units(&a, m->ctas, m->plan.tc_spread, tc_digits_ahead(m->max_terms, a.tc_rot_bytes != 0));
         a.n_units = a.n_blocks * a.units_per_block;
         a.zero_per_unit = (a.zero_slices + a.units_per_block - 1) / a.units_per_block;
     }

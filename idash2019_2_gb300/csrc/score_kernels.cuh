@@ -157,6 +157,8 @@ cudaError_t launch_finalize(const FinalizeArgs &a, cudaStream_t stream);
 // largest padded K is max_k_pad, its launch (grid = ctas, one per SM at
 // most), and the one-off shared-memory attribute.
 size_t tc_smem_bytes(uint32_t max_k_pad, bool rotated);
+// Whether the next unit's coefficient digits are loaded beside the current ones.
+bool tc_digits_ahead(uint32_t max_k_pad, bool rotated);
 cudaError_t launch_score_tc(const ScoreArgs &a, uint32_t ctas, cudaStream_t stream);
 cudaError_t configure_tc_kernel(size_t max_smem);
 

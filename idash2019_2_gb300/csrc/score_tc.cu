@@ -885,6 +885,11 @@ size_t tc_smem_bytes(uint32_t max_k_pad, bool rotated) {
     return x ? x->smem(max_k_pad, rotated) : SIZE_MAX;
 }
 
+bool tc_digits_ahead(uint32_t max_k_pad, bool rotated) {
+    const TcShape *x = tc_shape(max_k_pad, rotated);
+    return x && x->a_stages > 1;
+}
+
 cudaError_t configure_tc_kernel(size_t max_smem) {
     for (auto *fn : {k_score_tc<2, 2, 2, 1>, k_score_tc<2, 2, 2, 2>, k_score_tc<1, 3, 4, 1>, k_score_tc<1, 3, 4, 2>,
                      k_score_tc<1, 2, 4, kTcRotProducers, true>}) {
