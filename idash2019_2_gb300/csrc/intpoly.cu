@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyA
         const uint32_t q = warp / (kConsumers / 64), pt = tid % (kConsumers / 2);  // prime, points 4 pt ..
         const uint32_t p = q ? a.k.p[1] : a.k.p[0], pinv = q ? a.k.pinv[1] : a.k.pinv[0];
         const int32_t r1 = q ? a.k.r1[1] : a.k.r1[0];
+        // A lane that gives up exits; the warp's barriers are for the others.
         uint32_t s = q, parity = 0;  // the prime's stages in turn: q, q + 2, ...
         const uint32_t base = stage0 + 16 * pt;
         for (uint32_t turn = 0;;) {
@@ -511,7 +512,8 @@ __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyA
         // ----------------------------------------------------------- producers
         // Lookups run ahead of the copies: a group's outputs two groups, its
         // terms one, a row one step.  The warp runs the loop whole and one
-        // thread issues, so that addresses stay in uniform registers.
+        // thread issues, so that addresses stay in uniform registers; each lane
+        // leaves by its own verdict, as nothing in the loop waits for the others.
         const uint32_t q = warp - (kConsumers / 32 + kIpEpiWarps);
         const bool leader = elect_one();
         uint64_t g = a.group_begin + blockIdx.x;
@@ -558,7 +560,6 @@ __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyA
                         mbar_arrive(&sh.full[s]);
                     }
                 }
-                __syncwarp();
                 w += 2 * w_bytes;
                 ++issued;
                 s += 2;
@@ -572,7 +573,7 @@ __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyA
             members = next_members;
             row = next_row;
         }
-        if (!ok && lane == 0) {
+        if (!ok && leader) {
             // the consumers stopped: let the copies still in flight land
             constexpr uint32_t kMine = kScoreStages / 2;
             for (uint32_t k = issued > kMine ? issued - kMine : 0; k < issued; ++k)

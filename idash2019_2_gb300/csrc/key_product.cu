@@ -283,6 +283,8 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
         }
     } else if (warp >= kMmaWarp) {
         // ----------------------------------------------------------------- MMA
+        // Each lane leaves by its own verdict: nothing in the loop waits for the
+        // other lanes.
         const bool leader = elect_one();
         const uint32_t t = warp - kMmaWarp, d = tmem + t * kTileMax;
         const uint64_t a_desc = umma_desc(smem_addr(stages), kGroupBytes, 128);
@@ -310,7 +312,6 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
                     umma_commit(&sh.a_empty[s]);
                     if (c + 1 == n_chunks) umma_commit(&sh.acc_full[t]);
                 }
-                __syncwarp();
                 b += (kChunkWords / 8) * (128 / 16);
                 if (++s == n_stages) {
                     s = 0;

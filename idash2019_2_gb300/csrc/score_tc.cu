@@ -213,6 +213,7 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // `bar`'s phase also waits for this thread's cp.async so far.
 __device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
     asm volatile("cp.async.mbarrier.arrive.shared.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
@@ -472,18 +473,31 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
         fetch_rows();
         fetch_header();
         Ring rr, last;
-        bool ok = true, any = false;
-        for (Units w(a); ok && w.valid(a); w.next(a)) {
+        bool any = false;
+        // Lets the copies land: this warp's last ones (immediate when nothing
+        // aborted; every earlier one was waited for by way of its stage's
+        // converters or is behind one of these).
+        auto land = [&]() {
+            if (leader)
+                for (uint32_t s = me; s < a.tc_raw_stages; s += kProducers) {
+                    // the stage's last phase that this warp filled
+                    const uint32_t filled = last.round + (s <= last.s ? 1u : 0u);
+                    if (any && filled) mbar_wait_bounded(&sh.raw_full[s], (filled - 1) & 1u, nullptr);
+                }
+            cp_async_wait_all();
+        };
+        for (Units w(a); w.valid(a); w.next(a)) {
             const Rows x = next;
             fetch_rows();
             fetch_header();
-            // rows as held at a.in; 0, reported, for one outside it
+            // rows as held at a.in; 0, reported, for one outside it (and 0 past the
+            // block's slots: whatever lanes are left copy rows inside the input)
             __syncwarp();
 #pragma unroll
             for (uint32_t c = 0; c < kMaxChunks; ++c) {
                 uint32_t r = x.row[c] - a.row_base;
-                if (kChunk * c + lane < x.n_slots && r >= a.n_rows) {
-                    report_error(a.err, kDevBadIndex);
+                if (r >= a.n_rows) {
+                    if (kChunk * c + lane < x.n_slots) report_error(a.err, kDevBadIndex);
                     r = 0;
                 }
                 rows[kChunk * c + lane] = r;
@@ -497,7 +511,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
             const uint32_t boxes = __ballot_sync(0xFFFFFFFFu, n_here && a.tc_use_map && ((x.runs >> lane) & 1u) &&
                                                                   first < a.n_rows && n_here <= a.n_rows - first);
             const uint32_t s1 = w.s1(a);
-            for (uint32_t sl = w.s0(a); ok && sl < s1; ++sl) {
+            for (uint32_t sl = w.s0(a); sl < s1; ++sl) {
                 const uint32_t c0 = sl * kN;
 #pragma unroll 1
                 for (uint32_t c = 0; c < x.n_chunks; ++c) {
@@ -510,8 +524,10 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                     const int32_t r0 = int32_t(__shfl_sync(0xFFFFFFFFu, first, c));
                     uint64_t *full = &sh.raw_full[rr.s];
                     uint8_t *dst = raw + rr.s * kRawStageBytes;
-                    if (rr.round > 0 && !(ok = tc_wait(&sh.abort, &sh.raw_empty[rr.s], (rr.round - 1) & 1u, a.err)))
-                        break;
+                    if (rr.round > 0 && !tc_wait(&sh.abort, &sh.raw_empty[rr.s], (rr.round - 1) & 1u, a.err)) {
+                        land();
+                        return;  // the others of the warp do without this lane
+                    }
                     if ((boxes >> c) & 1u) {
                         if (leader) {
                             if (kRotated) rot.any[rr.s] = 0;
@@ -547,15 +563,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                 }
             }
         }
-        // Let the copies land: this warp's last ones (immediate when nothing
-        // aborted; every earlier one was waited for by way of its stage's
-        // converters or is behind one of these).
-        if (lane == 0)
-            for (uint32_t s = me; s < a.tc_raw_stages; s += kProducers) {
-                // the stage's last phase that this warp filled
-                const uint32_t filled = last.round + (s <= last.s ? 1u : 0u);
-                if (any && filled) mbar_wait_bounded(&sh.raw_full[s], (filled - 1) & 1u, nullptr);
-            }
+        land();
         __syncwarp();
     } else if (warp >= kConvWarp0) {
         // ---------------------------------------------------------- converters
@@ -640,6 +648,8 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
         }
     } else if (warp == kMmaWarp) {
         // ----------------------------------------------------------------- MMA
+        // Each lane leaves by its own verdict: nothing in the loop waits for the
+        // other lanes.
         Ring rd, ra, rt;
         bool ok = true;
         const bool leader = elect_one();
@@ -673,7 +683,6 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                             if (n == 1) umma_commit(&sh.a_empty[ra.s]);
                         }
                     }
-                    __syncwarp();
                     a0 += 512;
                     rd.next(a.tc_dig_stages);
                 }

@@ -1,0 +1,76 @@
+"""Bounded waits inside warps (csrc/waits.cuh), by reading the kernels' sources.
+Around an expiry the lanes of a warp can come to different verdicts on one wait,
+and a barrier, vote or shuffle of the whole warp then waits for a lane that has
+left the loop.  So a wait by a thread (tc_wait) is called only
+  - by one thread of a warp;
+  - or where a lane without what it waited for exits, which takes it out of the
+    barriers that follow;
+  - or in a loop without anything that waits for the other lanes."""
+import glob
+import os
+import re
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "idash2019_2_gb300", "csrc")
+WARP_WIDE = r"_sync\(|__syncwarp|__syncthreads|tc_warp_wait|tc_team_|load_rows\(|load_rotated<"
+
+
+def _code(path):
+    return re.sub(r"//[^\n]*|\"(\\.|[^\"\\\n])*\"", "", open(path).read())
+
+
+def _close(text, at, opening, closing):
+    """Position after the bracket that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += (text[i] == opening) - (text[i] == closing)
+        if depth == 0:
+            return i + 1
+    raise AssertionError("unbalanced")
+
+
+def _blocks_around(text, at):
+    """(header, body) of the braces open at position `at`, outermost first."""
+    stack = []
+    for i, ch in enumerate(text[:at]):
+        if ch == "{":
+            stack.append(i)
+        elif ch == "}":
+            stack.pop()
+    headers = []
+    for i in stack:
+        j = i - 1  # back to the end of the statement before the header; `for (;;)` has some inside
+        depth = 0
+        while j >= 0 and not (depth == 0 and text[j] in ";{}"):
+            depth += (text[j] == ")") - (text[j] == "(")
+            j -= 1
+        headers.append((text[j + 1:i].strip(), text[i:_close(text, i, "{", "}")]))
+    return headers
+
+
+def _exits(text, at):
+    """Whether the `if` whose condition holds position `at` ends the thread."""
+    start = max(text.rfind(c, 0, at) for c in ";{}") + 1
+    head = re.match(r"\s*(?:else\s+)?if \(", text[start:])
+    if not head:
+        return False
+    after = text[_close(text, start + head.end() - 1, "(", ")"):].lstrip()
+    return bool(re.match(r"return;|\{[^{}]*\breturn;\s*\}", after))
+
+
+def _alone(text, at):
+    blocks = _blocks_around(text, at)
+    if any(re.search(r"if \(lane == 0\)$", h) for h, _ in blocks) or _exits(text, at):
+        return True
+    loops = [body for h, body in blocks if re.search(r"\bfor \(", h)]
+    return bool(loops) and not re.search(WARP_WIDE, loops[0])
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cu"))), ids=os.path.basename)
+def test_no_lane_is_waited_for_after_it_gave_up(path):
+    text = _code(path)
+    for m in re.finditer(r"\btc_wait\(", text):
+        assert _alone(text, m.start()), (path, text[max(0, m.start() - 80):m.end() + 80])
