@@ -363,7 +363,7 @@ __device__ __forceinline__ void ip_accumulate(int64_t (&acc)[kGroupMax][2][4], u
 // both primes' copies and each output's sums reading the input transform anew.
 // Waiting consumers poll each for itself: meeting at a named barrier cost 8%.
 // Every wait is bounded and ends early once another role gave up; the producers
-// let their copies in flight land before they return.
+// let their copies in flight land before they return, however they came there.
 __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyArgs a) {
     extern __shared__ __align__(1024) uint8_t ip_smem[];
     constexpr uint32_t N = kIpN;  // a.N, checked on the host
@@ -573,8 +573,8 @@ __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyA
             members = next_members;
             row = next_row;
         }
-        if (!ok && leader) {
-            // the consumers stopped: let the copies still in flight land
+        if (leader) {
+            // let the last copies land, also when the consumers give up once all are issued
             constexpr uint32_t kMine = kScoreStages / 2;
             for (uint32_t k = issued > kMine ? issued - kMine : 0; k < issued; ++k)
                 mbar_wait_bounded(&sh.full[q + 2 * (k % kMine)], (k / kMine) & 1u, nullptr);

@@ -74,3 +74,13 @@ def test_no_lane_is_waited_for_after_it_gave_up(path):
     text = _code(path)
     for m in re.finditer(r"\btc_wait\(", text):
         assert _alone(text, m.start()), (path, text[max(0, m.start() - 80):m.end() + 80])
+
+
+@pytest.mark.parametrize("name", ["score_tc.cu", "key_product.cu", "intpoly.cu"])
+def test_copies_in_flight_land_on_every_way_out(name):
+    """A role's wait for its own copies (the one that reports no error) does not
+    depend on its verdict: other roles may give up after it has issued all."""
+    text = _code(os.path.join(CSRC, name))
+    for m in re.finditer(r"\bmbar_wait_bounded\([^;]*nullptr\);", text):
+        for header, _ in _blocks_around(text, m.start()):
+            assert not re.search(r"if \(.*!\s*ok\b", header), (name, header)
