@@ -301,6 +301,11 @@ __device__ __forceinline__ void fold(int64_t &T, int32_t r1) {
     T = int64_t((uint64_t(hi) << 32) | lo);
 }
 
+// The epilogue's wait for a group's sums is as long as the group: up to 2^20 row
+// steps, 0.44 s of the second that other waits have.  So its limit grows by this
+// for each step (a step takes some 1,100 cycles with all SMs at work).
+constexpr long long kStepLimitCycles = 1 << 14;
+
 // Stage layout, for one prime: the input row's transform (2 polynomials), then
 // the weights' of up to kGroupMax outputs at the same term, N words each.
 constexpr uint32_t kStageWords = (2 + kGroupMax) * kIpN;
@@ -453,11 +458,13 @@ __global__ void __launch_bounds__(kScoreBlock, 1) k_intpoly_score(const IntpolyA
         uint32_t turn = 0;
         uint64_t g = a.group_begin + blockIdx.x;
         for (; g < a.group_end; g += gridDim.x, ++turn) {
-            const uint64_t o = a.group_first[g] + m;
+            const uint64_t o0 = a.group_first[g], o = o0 + m;
             const bool mine = o < a.group_first[g + 1] && o >= a.out_begin && o < a.out_end;
             const uint32_t add = mine && poly == 1 && a.bias ? uint32_t(a.bias[o]) * uint32_t(a.one) : 0u;
             const bool polls = m == 0 && poly == 0 && lane == 0;
-            if (!tc_team_wait<32 * kIpEpiWarps>(1, polls, &sh.abort, &sh.sums_full, turn & 1u, a.err)) return;
+            const long long limit =
+                kWaitLimitCycles + (polls ? (long long)(a.term_ptr[o0 + 1] - a.term_ptr[o0]) * kStepLimitCycles : 0);
+            if (!tc_team_wait<32 * kIpEpiWarps>(1, polls, &sh.abort, &sh.sums_full, turn & 1u, a.err, limit)) return;
             if (!mine) {
                 if (lane == 0) mbar_arrive(&sh.sums_empty);
                 continue;

@@ -16,7 +16,8 @@ namespace idash {
 //     have are undefined: no address may depend on them).
 // (One verdict for all by a shuffle or vote after each wait: 0.2 to 2.6% of a
 // scoring pass with TRLWE rows, 1.5 to 5% with LWE rows.)
-__device__ __forceinline__ bool tc_wait(uint32_t *abort, uint64_t *bar, uint32_t parity, uint32_t *err) {
+__device__ __forceinline__ bool tc_wait(uint32_t *abort, uint64_t *bar, uint32_t parity, uint32_t *err,
+                                        long long limit = kWaitLimitCycles) {
     if (mbar_try_wait(bar, parity)) return true;
     volatile uint32_t *flag = abort;
     const long long t0 = clock64();
@@ -27,7 +28,7 @@ __device__ __forceinline__ bool tc_wait(uint32_t *abort, uint64_t *bar, uint32_t
         for (int i = 0; i < 8; ++i)
             if (mbar_try_wait_sleep(bar, parity, 20000u)) return true;
         if (*flag != 0) return false;
-        if (clock64() - t0 > kWaitLimitCycles) {
+        if (clock64() - t0 > limit) {
             report_error(err, kDevTimeout);
             *flag = 1u;
             return false;
@@ -63,8 +64,8 @@ __device__ __forceinline__ bool tc_team_and(uint32_t id, bool ok) {
 
 template <int kThreads>
 __device__ __forceinline__ bool tc_team_wait(uint32_t id, bool polls, uint32_t *abort, uint64_t *bar, uint32_t parity,
-                                             uint32_t *err) {
-    return tc_team_and<kThreads>(id, !polls || tc_wait(abort, bar, parity, err));
+                                             uint32_t *err, long long limit = kWaitLimitCycles) {
+    return tc_team_and<kThreads>(id, !polls || tc_wait(abort, bar, parity, err, limit));
 }
 
 }  // namespace idash

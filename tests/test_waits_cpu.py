@@ -9,6 +9,8 @@ left the loop.  So a wait by a thread (tc_wait) is called only
 import glob
 import os
 import re
+import shutil
+import subprocess
 
 import pytest
 
@@ -84,3 +86,48 @@ def test_copies_in_flight_land_on_every_way_out(name):
     for m in re.finditer(r"\bmbar_wait_bounded\([^;]*nullptr\);", text):
         for header, _ in _blocks_around(text, m.start()):
             assert not re.search(r"if \(.*!\s*ok\b", header), (name, header)
+
+
+LIMITS = """#include <cstdint>
+#define __device__
+#define __forceinline__ inline
+static long long now, done;  // the clock, and when the phase completes
+inline long long clock64() { return now; }
+inline uint32_t __shfl_sync(uint32_t, uint32_t v, int) { return v; }
+namespace idash {
+constexpr long long kWaitLimitCycles = 2000000000ll;
+constexpr uint32_t kDevTimeout = 2;
+inline void report_error(uint32_t *err, uint32_t code) { *err = code; }
+inline bool mbar_try_wait(uint64_t *, uint32_t) { return now >= done; }
+inline bool mbar_try_wait_sleep(uint64_t *, uint32_t, uint32_t) { now += 40000; return now >= done; }
+}
+#include "waits.cuh"
+using namespace idash;
+int main() {
+    // a phase after three seconds: late for a hand-off, in time for 2^20 steps
+    for (int grown = 0; grown < 2; ++grown) {
+        uint32_t abort = 0, err = 0;
+        uint64_t bar = 0;
+        now = 0;
+        done = 6000000000ll;
+        const long long limit = kWaitLimitCycles + (grown ? (1ll << 20) * (1 << 14) : 0);
+        if (tc_wait(&abort, &bar, 0, &err, limit) != (grown == 1) || err != (grown ? 0u : kDevTimeout)) return 1;
+    }
+    return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_a_groups_sums_are_waited_for_as_long_as_the_group(tmp_path):
+    """The wait for an integer-polynomial group's sums lasts as long as its row
+    steps (up to 2^20): its limit grows with them."""
+    shutil.copy(os.path.join(CSRC, "waits.cuh"), tmp_path / "waits.cuh")
+    (tmp_path / "common.cuh").write_text("#pragma once\n")
+    (tmp_path / "main.cpp").write_text(LIMITS)
+    subprocess.run(["g++", "-std=c++17", "-I", str(tmp_path), "-o", str(tmp_path / "limits"), str(tmp_path / "main.cpp")],
+                   check=True)
+    assert subprocess.run([str(tmp_path / "limits")], timeout=60).returncode == 0
+    text = _code(os.path.join(CSRC, "intpoly.cu"))
+    assert re.search(r"limit\s*=\s*kWaitLimitCycles \+ \(polls \? [^;]*kStepLimitCycles", text)
+    assert re.search(r"sh\.sums_full, turn & 1u, a\.err, limit\)", text)
