@@ -21,6 +21,7 @@
 // (Longa & Naehrig, CANS 2016).
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "capi_internal.hpp"
@@ -663,7 +664,10 @@ struct IntpolyModel {
     uint2 *d_itw = nullptr;  // inverse twiddles and quotients [2][N]
     uint32_t *d_c_hat = nullptr;
     uint64_t c_hat_rows = 0;
+    std::mutex order;              // calls take their turns (IntpolyTurn)
+    cudaEvent_t used = nullptr;    // the last call's kernels are done
     ~IntpolyModel() {
+        if (used) cudaEventDestroy(used);
         cudaFree(d_term_ptr);
         cudaFree(d_term_row);
         cudaFree(d_slot);
@@ -681,6 +685,30 @@ namespace {
 uint32_t ntt_grid(uint64_t n_polys, uint32_t per_sm, const idash_ctx *ctx) {
     return uint32_t(std::min<uint64_t>(n_polys, uint64_t(ctx->sm_count) * per_sm));
 }
+
+// A call's turn at the model's transforms, of which there is one set (d_w_hat,
+// d_c_hat): its kernels follow those of the call before, whatever the streams.
+// Captured into a caller's graph, the wait and the record are nodes of it, and a
+// replay takes its turn like a call.
+class IntpolyTurn {
+    IntpolyModel &ip;
+    cudaStream_t stream;
+    std::lock_guard<std::mutex> lock;
+    bool captured = false;
+
+  public:
+    IntpolyTurn(IntpolyModel &ip_, cudaStream_t s) : ip(ip_), stream(s), lock(ip_.order) {}
+    cudaError_t begin() {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        const cudaError_t e = cudaStreamIsCapturing(stream, &status);
+        if (e != cudaSuccess) return e;
+        captured = status == cudaStreamCaptureStatusActive;
+        return cudaStreamWaitEvent(stream, ip.used, captured ? cudaEventWaitExternal : cudaEventWaitDefault);
+    }
+    cudaError_t end() {
+        return cudaEventRecordWithFlags(ip.used, stream, captured ? cudaEventRecordExternal : cudaEventRecordDefault);
+    }
+};
 
 // The transforms of terms [t0, t0 + n), whose polynomials are at w.
 cudaError_t launch_ntt_model(const IntpolyModel &ip, const int16_t *w, uint64_t t0, uint64_t n, idash_ctx *ctx,
@@ -752,7 +780,7 @@ extern "C" idash_status idash_model_intpoly(idash_ctx *ctx, idash_model **model,
         idash_model_free(m);
         return s;
     };
-    idash_status s = IDASH_OK;
+    idash_status s = ctx->check_cuda(cudaEventCreateWithFlags(&ip.used, cudaEventDisableTiming), "cudaEventCreate");
     auto up = [&](void **dst, const void *src, size_t bytes, const char *what) {
         if (s != IDASH_OK) return;
         s = ctx->check_cuda(cudaMalloc(dst, std::max<size_t>(bytes, 16)), what);
@@ -821,7 +849,11 @@ extern "C" idash_status idash_model_intpoly_set_weights(idash_model *m, const in
     if (ip.n_terms == 0) return IDASH_OK;
     if (!d_term_poly) return IDASH_ERR_INVALID_ARGUMENT;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-    return ctx->check_cuda(launch_ntt_model(ip, d_term_poly, 0, ip.n_terms, ctx, st), "k_ntt launch");
+    IntpolyTurn turn(ip, st);
+    idash_status s = ctx->check_cuda(turn.begin(), "wait for the model's last call");
+    if (s == IDASH_OK) s = ctx->check_cuda(launch_ntt_model(ip, d_term_poly, 0, ip.n_terms, ctx, st), "k_ntt launch");
+    if (s == IDASH_OK) s = ctx->check_cuda(turn.end(), "record the model's last call");
+    return s;
 }
 
 extern "C" idash_status idash_score_intpoly_device(idash_model *m, const void *d_in, const idash_row_layout *il,
@@ -840,7 +872,9 @@ extern "C" idash_status idash_score_intpoly_device(idash_model *m, const void *d
         return ctx->fail(IDASH_ERR_INVALID_ARGUMENT, "row layout: stride or alignment");
     if (out_begin == out_end) return IDASH_OK;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-    idash_status s = IDASH_OK;
+    IntpolyTurn turn(ip, st);
+    idash_status s = ctx->check_cuda(turn.begin(), "wait for the model's last call");
+    if (s != IDASH_OK) return s;
     if (ip.c_hat_rows < ip.n_rows) {
         if ((s = ctx->check_cuda(cudaStreamSynchronize(st), "sync before growing C^")) != IDASH_OK) return s;
         cudaFree(ip.d_c_hat);
@@ -890,6 +924,7 @@ extern "C" idash_status idash_score_intpoly_device(idash_model *m, const void *d
     const uint32_t grid = uint32_t(std::min<uint64_t>(a.group_end - a.group_begin, ctx->sm_count));
     k_intpoly_score<<<grid, kScoreBlock, kIpScoreSmem, st>>>(a);
     s = ctx->check_cuda(cudaGetLastError(), "k_intpoly_score launch");
+    if (s == IDASH_OK) s = ctx->check_cuda(turn.end(), "record the model's last call");
     if (s == IDASH_OK) ctx->stats.kernel_launches += 2;
     return s;
 }

@@ -322,7 +322,10 @@ idash_status idash_model_intpoly(idash_ctx *ctx, idash_model **model, const idas
  * then undefined until replaced again. */
 idash_status idash_model_intpoly_set_weights(idash_model *model, const int16_t *d_term_poly, void *stream);
 /* Scores outputs [out_begin, out_end) (output o -> row o - out_begin) from
- * the n_in_rows input TRLWE rows at d_in.  Asynchronous on `stream`. */
+ * the n_in_rows input TRLWE rows at d_in.  Asynchronous on `stream`.  Calls on
+ * one model (this one and idash_model_intpoly_set_weights) take effect in the
+ * order they are made, on whatever streams: each waits on the device for the
+ * one before. */
 idash_status idash_score_intpoly_device(idash_model *model, const void *d_in, const idash_row_layout *in_layout,
                                         uint64_t out_begin, uint64_t out_end, void *d_out,
                                         const idash_row_layout *out_layout, void *stream);
