@@ -327,7 +327,8 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
         // ------------------------------------------------------------ epilogue
         constexpr uint32_t kMagicSum = kMagicBits + (kMagicBits << 11) + (kMagicBits << 22);
         const uint32_t half = warp / 4, quadrant = warp % 4, c_lane = 2 * (lane % 4);
-        for (uint64_t it = 0; it < 2 * my_items; ++it) {
+        uint64_t it = 0;
+        for (; it < 2 * my_items; ++it) {
             const uint64_t i = it / 2, item = blockIdx.x + i * gridDim.x;
             const uint32_t t = it % 2;
             const uint64_t row = (item / a.pairs) * kRows + 8 * quadrant + lane / 4;
@@ -390,12 +391,31 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
             }
             if (first >= last && lane == 0) mbar_arrive(&sh.acc_empty[t]);
         }
+        // given up: no body stays without its product
+        for (; !kScores && it < 2 * my_items; ++it) {
+            const uint64_t item = blockIdx.x + (it / 2) * gridDim.x;
+            const uint64_t row = (item / a.pairs) * kRows + 8 * quadrant + lane / 4;
+            uint32_t n0, w;
+            tile_of(item, it % 2, n0, w);
+            if (row >= a.n_rows) continue;
+            uint32_t *body = reinterpret_cast<uint32_t *>(const_cast<uint8_t *>(kp_row(a, row))) + N;
+            const uint32_t middle = (w / 2 + 15u) & ~15u, end = min(n0 + (half ? w : middle), a.n_coef);
+            for (uint32_t j = n0 + (half ? middle : 0u) + lane % 4; j < end; j += 4) body[j] = 0;
+        }
     }
 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     if (warp == kMmaWarp) tmem_dealloc(tmem, 2 * kTileMax);
+}
+
+// The bodies' coefficients [0, n_coef) to zero, a CTA to a row in turn.
+__global__ void k_clear_bodies(const __grid_constant__ KeyProductArgs a) {
+    for (uint64_t r = blockIdx.x; r < a.n_rows; r += gridDim.x) {
+        uint32_t *body = reinterpret_cast<uint32_t *>(const_cast<uint8_t *>(kp_row(a, r))) + a.N;
+        for (uint32_t j = threadIdx.x; j < a.n_coef; j += blockDim.x) body[j] = 0;
+    }
 }
 
 }  // namespace
@@ -419,7 +439,10 @@ cudaError_t launch_key_product(KeyProductArgs a, int sm_count, cudaStream_t s) {
     a.vec_scores = ((reinterpret_cast<uintptr_t>(a.scores) | (uint64_t(a.n_coef) * 4)) & 7u) == 0;
     auto *fn = a.scores ? k_key_product<true> : k_key_product<false>;
     fn<<<uint32_t(std::min<uint64_t>(a.items, uint64_t(sm_count))), kKpThreads, kp_smem(a.N), s>>>(a);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess && !a.scores)
+        k_clear_bodies<<<uint32_t(std::min<uint64_t>(a.n_rows, uint64_t(sm_count) * 8)), 256, 0, s>>>(a);
+    return e;
 }
 
 cudaError_t configure_key_product() {
@@ -428,7 +451,8 @@ cudaError_t configure_key_product() {
                                                    int(std::max(kp_smem(1024), kp_smem(kKeyMaxN))));
         if (e != cudaSuccess) return e;
     }
-    return cudaSuccess;
+    cudaFuncAttributes loaded{};  // now, not when something else has failed
+    return cudaFuncGetAttributes(&loaded, k_clear_bodies);
 }
 
 }  // namespace idash

@@ -36,7 +36,9 @@ struct KeyProductArgs {
 };
 
 // scores non-null: scores[r * n_coef + j] = float((b - a*s)[j] / 2^32).
-// scores null: b[j] += (a*s)[j] in place.
+// scores null: b[j] += (a*s)[j] in place.  Bodies that the product does not get
+// into (the launch fails, or a wait on the device expires) are cleared: they
+// hold messages.
 cudaError_t launch_key_product(KeyProductArgs a, int sm_count, cudaStream_t s);
 
 // Allows the kernels their shared memory (once per device, before any launch or capture).

@@ -417,7 +417,10 @@ idash_status idash_cloud_files(int device, const char *params_file, const char *
  * generator keyed by `seed` (a statistical generator, as TFHE's is, not a
  * cryptographic one).  d_noise (optional, n_rows * N int32) receives e.
  * key: N integer coefficients in host memory; N a power of two in [4, 2048].
- * Asynchronous on `stream` once the key has been staged. */
+ * Asynchronous on `stream` once the key has been read.  Read no row before the
+ * call's work on `stream` is done: bodies are complete only then.  After an error,
+ * from this call or (IDASH_ERR_DEVICE_TIMEOUT) from the synchronising one, the
+ * rows are not ciphertexts; bodies without their product are cleared. */
 typedef struct {
     uint32_t N, k;          /* k must be 1 */
     uint32_t num_samples;   /* NUM_SAMPLES */
