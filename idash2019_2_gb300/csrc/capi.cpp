@@ -304,6 +304,35 @@ void block_range(const idash_model *m, uint32_t p, uint64_t o_begin, uint64_t o_
     *hi = uint32_t(last - B.begin());
 }
 
+// The input rows [*row_begin, *row_end) that outputs [out_begin, out_end) need: all
+// rows of their blocks, or (where the plan knows them, and not asked for whole
+// blocks) those that the outputs read themselves.
+void rows_read(const idash_model *m, uint64_t out_begin, uint64_t out_end, bool whole_blocks, uint64_t *row_begin,
+               uint64_t *row_end) {
+    uint64_t lo = UINT64_MAX, hi = 0;
+    auto reads = [&](uint64_t first, uint64_t end) {
+        lo = std::min(lo, first);
+        hi = std::max(hi, end);
+    };
+    const auto &own = m->plan.tc_out_rows;
+    for (uint32_t p = 0; p < n_phases(m); ++p) {
+        uint32_t b_lo, b_hi;
+        block_range(m, p, out_begin, out_end, &b_lo, &b_hi);
+        for (uint32_t b = b_lo; b < b_hi; ++b) {
+            const PlanBlock &block = m->plan.blocks[b];
+            if (block.n_slots == 0) continue;
+            if (own.empty() || whole_blocks || (block.out_lo >= out_begin && block.out_hi <= out_end)) {
+                reads(m->plan.block_min_row[b], uint64_t(m->plan.block_max_row[b]) + 1);
+                continue;
+            }
+            for (uint64_t o = std::max<uint64_t>(block.out_lo, out_begin); o < std::min<uint64_t>(block.out_hi, out_end); ++o)
+                if (own[o].second) reads(own[o].first, own[o].second);
+        }
+    }
+    *row_begin = lo == UINT64_MAX ? 0 : lo;
+    *row_end = hi;
+}
+
 // Launches the scoring kernel over every phase's blocks that touch outputs
 // [o_lo, o_hi), phase by phase on `s` (later phases add to what earlier ones
 // wrote); args(b_lo, b_hi) builds one launch's arguments.
@@ -1074,19 +1103,7 @@ idash_status idash_score_trlwe_host(idash_model *m, const void *h_in, const idas
 idash_status idash_model_input_rows(const idash_model *m, uint64_t out_begin, uint64_t out_end, uint64_t *row_begin,
                                     uint64_t *row_end) {
     if (!m || !row_begin || !row_end || out_begin > out_end || out_end > m->n_out) return IDASH_ERR_INVALID_ARGUMENT;
-    uint64_t lo = UINT64_MAX, hi = 0;
-    for (uint32_t p = 0; p < n_phases(m); ++p) {
-        uint32_t b_lo, b_hi;
-        block_range(m, p, out_begin, out_end, &b_lo, &b_hi);
-        for (uint32_t b = b_lo; b < b_hi; ++b) {
-            if (m->plan.blocks[b].n_slots == 0) continue;
-            lo = std::min<uint64_t>(lo, m->plan.block_min_row[b]);
-            hi = std::max<uint64_t>(hi, uint64_t(m->plan.block_max_row[b]) + 1);
-        }
-    }
-    if (lo == UINT64_MAX) lo = hi = 0;
-    *row_begin = lo;
-    *row_end = hi;
+    rows_read(m, out_begin, out_end, false, row_begin, row_end);
     return IDASH_OK;
 }
 
@@ -1112,10 +1129,14 @@ idash_status score_trlwe_range(idash_model *m, uint64_t out_begin, uint64_t out_
     if (s == IDASH_OK) s = check_layout(ctx, d_out, ol, payload, true);
     if (s != IDASH_OK) return s;
     if (out_begin == out_end) return IDASH_OK;
-    uint64_t r_lo, r_hi;
-    idash_model_input_rows(m, out_begin, out_end, &r_lo, &r_hi);
-    if (r_hi > r_lo && (r_lo < in_row_base || r_hi > in_row_base + n_in_rows))
+    auto lacks = [&](bool whole_blocks) {
+        uint64_t lo, hi;
+        rows_read(m, out_begin, out_end, whole_blocks, &lo, &hi);
+        return hi > lo && (lo < in_row_base || hi > in_row_base + n_in_rows);
+    };
+    if (lacks(false))
         return ctx->fail(IDASH_ERR_INDEX, "the outputs read input rows outside [in_row_base, in_row_base + n_in_rows)");
+    const bool partial = !m->plan.tc_out_rows.empty() && lacks(true);
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
     const uint8_t *in = static_cast<const uint8_t *>(d_in);
     uint8_t *out = static_cast<uint8_t *>(d_out);
@@ -1132,6 +1153,7 @@ idash_status score_trlwe_range(idash_model *m, uint64_t out_begin, uint64_t out_
         a.row_base = uint32_t(in_row_base);
         a.n_rows = uint32_t(n_in_rows);
         if (num_samples) a.num_samples = num_samples;
+        a.tc_rows_partial = partial;
         if (fuse) {
             a.digest = reinterpret_cast<unsigned long long *>(digest);
             a.digest_base = digest_base;

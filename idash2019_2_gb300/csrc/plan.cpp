@@ -417,11 +417,17 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
     plan->tc_producers = 4 * scattered > chunks ? kTcMaxProducers : 1;
     uint32_t rotations = 0;  // all of them, or-ed
     for (uint64_t k : nm.nkey) rotations |= uint32_t(k);
-    if (rotations) {
+    if (in.form == Form::kTrlwe && in.num_regions > 1) {
         // a tile of columns is inside one polynomial, and a rotation a mask
         if (in.N % 64 != 0 || (in.N & (in.N - 1)) != 0) return "the tensor-core plan rotates rows of 2^k >= 64 coefficients";
         plan->tc_rot_bytes = rotations & 1u ? 4 : rotations & 2u ? 8 : 16;
         plan->tc_producers = kTcRotProducers;
+        plan->tc_out_rows.resize(n_out);
+        for (uint64_t o = 0; o < n_out; ++o) {
+            // keys in order: the first row and the last
+            const uint64_t t0 = nm.nptr[o], t1 = nm.nptr[o + 1];
+            if (t0 < t1) plan->tc_out_rows[o] = {uint32_t(nm.nkey[t0] >> 32), uint32_t(nm.nkey[t1 - 1] >> 32) + 1};
+        }
     }
     // a slice of K rows costs about K + 60 (the epilogue)
     double sum = 0, squares = 0;

@@ -16,6 +16,7 @@
 
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace idash {
@@ -114,7 +115,12 @@ struct Plan {
     std::vector<TcOut> tc_out;
     uint32_t tc_producers = 1;  // kTcMaxProducers where more than a quarter of the 32-row chunks are scattered rows
     double tc_spread = 0;       // standard deviation of a slice's cost over the blocks, in mean costs
-    uint32_t tc_rot_bytes = 0;  // rotated rows: the largest copy (4, 8 or 16 bytes) that every rotation keeps aligned; 0: none
+    // Several regions to a row: the largest copy (4, 8 or 16 bytes) that every
+    // rotation keeps aligned (0: one region); and per output the input rows
+    // [first, second) that it reads, as a range of outputs need not bring all of
+    // its blocks' rows.
+    uint32_t tc_rot_bytes = 0;
+    std::vector<std::pair<uint32_t, uint32_t>> tc_out_rows;
 };
 
 // Tensor-core plans (build_tc_plan).  A block is up to kTcRows consecutive

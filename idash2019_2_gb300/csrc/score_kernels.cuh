@@ -73,6 +73,7 @@ struct ScoreArgs {
     uint32_t tc_a_max_bytes;      // shared-memory room for one block's digits
     uint32_t tc_producers;        // row-loading warps (Plan::tc_producers)
     uint32_t tc_rot_bytes;        // rotated slots (Plan::tc_rot_bytes)
+    uint32_t tc_rows_partial;     // with them: the input may lack rows that no output of [out_lo, out_hi) reads
     // with them, n_slices are those with a column that is not zeroed (from N +
     // region_size on); zero_slices follow them, zero_per_unit for each unit of a block
     uint32_t zero_slices, zero_per_unit;

@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
             head.next(a);
         };
         auto fetch_rows = [&]() {  // of the block header last read
-            next.n_slots = blk.n_slots;
+            next.n_slots = a.n_rows ? blk.n_slots : 0;
             next.runs = blk.term_begin;
             next.n_chunks = (blk.n_groups + kChunk - 1) / kChunk;
 #pragma unroll
@@ -491,13 +491,16 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
             fetch_rows();
             fetch_header();
             // rows as held at a.in; 0, reported, for one outside it (and 0 past the
-            // block's slots: whatever lanes are left copy rows inside the input)
+            // block's slots: whatever lanes are left copy rows inside the input).
+            // With tc_rows_partial a row outside is one that only outputs not
+            // wanted read, and any other does.
             __syncwarp();
 #pragma unroll
             for (uint32_t c = 0; c < kMaxChunks; ++c) {
                 uint32_t r = x.row[c] - a.row_base;
                 if (r >= a.n_rows) {
-                    if (kChunk * c + lane < x.n_slots) report_error(a.err, kDevBadIndex);
+                    if (kChunk * c + lane < x.n_slots && !(kRotated && a.tc_rows_partial))
+                        report_error(a.err, kDevBadIndex);
                     r = 0;
                 }
                 rows[kChunk * c + lane] = r;
@@ -924,8 +927,9 @@ cudaError_t launch_score_tc(const ScoreArgs &a_in, uint32_t ctas, cudaStream_t s
         return cudaErrorInvalidValue;
     TcMaps maps;
     std::memset(&maps, 0, sizeof(maps));
-    a.tc_use_map = encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, kChunk, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                   &maps.rows);
+    // (no boxes over rows that are not all there)
+    a.tc_use_map = !a.tc_rows_partial && encode_rows_map(a.in, a.row_words, a.n_rows, a.in_stride, kN, kChunk,
+                                                         CU_TENSOR_MAP_SWIZZLE_NONE, &maps.rows);
     a.tc_store_map = !a.out_row_map && a.out_lo >= a.out_row_base &&
                      encode_rows_map(a.out, a.row_words, a.out_hi - a.out_row_base, a.out_stride, 32, 32,
                                      CU_TENSOR_MAP_SWIZZLE_128B, &maps.out);
