@@ -306,9 +306,10 @@ void block_range(const idash_model *m, uint32_t p, uint64_t o_begin, uint64_t o_
 
 // The input rows [*row_begin, *row_end) that outputs [out_begin, out_end) need: all
 // rows of their blocks, or (where the plan knows them, and not asked for whole
-// blocks) those that the outputs read themselves.
-void rows_read(const idash_model *m, uint64_t out_begin, uint64_t out_end, bool whole_blocks, uint64_t *row_begin,
-               uint64_t *row_end) {
+// blocks) those that the outputs read themselves; with `variances`, those of
+// terms that cancel too.
+void rows_read(const idash_model *m, uint64_t out_begin, uint64_t out_end, bool whole_blocks, bool variances,
+               uint64_t *row_begin, uint64_t *row_end) {
     uint64_t lo = UINT64_MAX, hi = 0;
     auto reads = [&](uint64_t first, uint64_t end) {
         lo = std::min(lo, first);
@@ -329,6 +330,9 @@ void rows_read(const idash_model *m, uint64_t out_begin, uint64_t out_end, bool 
                 if (own[o].second) reads(own[o].first, own[o].second);
         }
     }
+    if (variances && m->plan.cancelled && !m->plan.var_ptr.empty())
+        for (uint64_t t = m->plan.var_ptr[out_begin]; t < m->plan.var_ptr[out_end]; ++t)
+            reads(m->plan.var_row[t], uint64_t(m->plan.var_row[t]) + 1);
     *row_begin = lo == UINT64_MAX ? 0 : lo;
     *row_end = hi;
 }
@@ -1103,7 +1107,7 @@ idash_status idash_score_trlwe_host(idash_model *m, const void *h_in, const idas
 idash_status idash_model_input_rows(const idash_model *m, uint64_t out_begin, uint64_t out_end, uint64_t *row_begin,
                                     uint64_t *row_end) {
     if (!m || !row_begin || !row_end || out_begin > out_end || out_end > m->n_out) return IDASH_ERR_INVALID_ARGUMENT;
-    rows_read(m, out_begin, out_end, false, row_begin, row_end);
+    rows_read(m, out_begin, out_end, false, true, row_begin, row_end);
     return IDASH_OK;
 }
 
@@ -1131,7 +1135,7 @@ idash_status score_trlwe_range(idash_model *m, uint64_t out_begin, uint64_t out_
     if (out_begin == out_end) return IDASH_OK;
     auto lacks = [&](bool whole_blocks) {
         uint64_t lo, hi;
-        rows_read(m, out_begin, out_end, whole_blocks, &lo, &hi);
+        rows_read(m, out_begin, out_end, whole_blocks, il->variance_offset >= 0 && ol->variance_offset >= 0, &lo, &hi);
         return hi > lo && (lo < in_row_base || hi > in_row_base + n_in_rows);
     };
     if (lacks(false))

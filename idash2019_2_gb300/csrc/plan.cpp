@@ -90,6 +90,8 @@ std::string normalise(const PlanInput &in, Plan *plan, Normalised *nm, bool *ind
             if (c != 0) {
                 nkey.push_back(tmp[i].first);
                 ncoef.push_back(c);
+            } else {
+                plan->cancelled = true;
             }
             i = j;
         }

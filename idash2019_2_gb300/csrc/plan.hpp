@@ -107,6 +107,9 @@ struct Plan {
     uint64_t n_terms_in = 0;       // CSR terms given
     uint64_t distinct_rows = 0;    // input rows read at least once
     uint32_t max_row_per_block_hint = 0;
+    // Some output has terms that cancel: their rows are in var_row (a variance
+    // counts each term) but in no block.
+    bool cancelled = false;
     std::vector<uint32_t> block_max_row;  // per block: largest input row read
     std::vector<uint32_t> block_min_row;  // per block: smallest input row read (0 if none)
     // Tensor-core plans only (build_tc_plan): per block, the coefficient

@@ -87,3 +87,44 @@ def test_outputs_without_terms_bring_no_row(ctx, oracle):
     m.free()
     d_in.free()
     d_out.free()
+
+
+@pytest.mark.parametrize("regions,size,kernel", [(1, 1024, 0), (1, 1024, 2), (3, 341, 0)])
+def test_variances_of_terms_that_cancel(ctx, oracle, regions, size, kernel):
+    """A feature whose coefficients cancel is read for its variance alone: a window
+    without its row is refused where variances are asked for, and taken where not."""
+    far = 3 * 50 if regions > 1 else 50  # region 0 of row 50
+    ptr, ns = np.array([0, 4, 5], np.uint64), size - 1
+    feat = np.array([0, regions, far, far, regions], np.uint32)
+    coef = np.array([3, 4, 7, -7, 2], np.int32)
+    n_rows = 60
+    rows = np.random.default_rng(2).integers(0, 2 ** 32, size=(n_rows, 2048), dtype=np.uint64).astype(np.uint32).view(np.int32)
+    var = np.arange(1.0, n_rows + 1.0)
+    rec = np.zeros((n_rows, gpu.RECORD_BYTES), np.uint8)
+    rec[:, 8:8200] = rows.view(np.uint8).reshape(n_rows, 8192)
+    rec[:, 8200:] = var[:, None].view(np.uint8)
+    want, _ = oracle.trlwe_score(ptr, feat, coef, rows, ns, regions, size)
+    ctx.set_option("kernel", kernel)
+    try:
+        m = gpu.TrlweModel(ctx, gpu.CSRModel(ptr, feat, coef), n_rows, ns, regions, size)
+    finally:
+        ctx.set_option("kernel", 0)
+    assert m.input_rows(0, 1) == (0, 51)
+    d_in, d_out = ctx.device_alloc(rec.nbytes + 16), ctx.device_alloc(2 * gpu.RECORD_BYTES + 16)
+    d_in.upload(rec, offset=8)
+    d_out.zero()
+    at = (d_in.ptr + 8, gpu.RECORD_IN, 0)
+    m.score_range(0, 1, 0, *at, 51, d_out.ptr + 8, gpu.RECORD_OUT)
+    ctx.sync()
+    got = d_out.download(nbytes=gpu.RECORD_BYTES, offset=8)
+    np.testing.assert_array_equal(got[8:8200].view(np.int32), want[0])
+    assert got[8200:].view(np.float64)[0] == 9 * 1.0 + 16 * 2.0 + 49 * 51.0 + 49 * 51.0
+    with pytest.raises(gpu.IdashError) as e:
+        m.score_range(0, 1, 0, *at, 2, d_out.ptr + 8, gpu.RECORD_OUT)
+    assert e.value.name == "IDASH_ERR_INDEX"
+    m.score_range(0, 1, 0, *at, 2, d_out.ptr, gpu.DENSE_TRLWE)
+    ctx.sync()
+    np.testing.assert_array_equal(d_out.download(nbytes=8192, dtype=np.int32), want[0])
+    m.free()
+    d_in.free()
+    d_out.free()
