@@ -91,7 +91,7 @@ __host__ __device__ constexpr uint32_t kp_table_bytes(uint32_t N) { return (2 * 
 // at least 120 KB, so that no second CTA (which would wait for this one's
 // tensor memory) fits on the SM
 constexpr size_t kp_smem(uint32_t N) { return kHeader + kp_table_bytes(N) + size_t(kp_stages(N)) * kStageBytes; }
-static_assert(kp_smem(64) > 120 * 1024, "one CTA per SM");
+static_assert(kp_smem(32) > 120 * 1024, "one CTA per SM");
 static_assert(kp_smem(1024) <= 227 * 1024 && kp_smem(kKeyMaxN) <= 227 * 1024, "shared memory");
 
 __device__ __forceinline__ const uint8_t *kp_row(const KeyProductArgs &a, uint64_t r) {
@@ -140,14 +140,16 @@ __device__ __forceinline__ uint32_t kp_entry(const uint32_t *key, uint32_t N, in
 }
 
 // kScores: decryption (scores from b - a*s), else b += a*s.
-template <bool kScores>
+// kHalf: N = 32, one chunk of which the first half is the row's words (told apart
+// at run time, the issuing loop made 1,000 coefficients 3% slower).
+template <bool kScores, bool kHalf>
 __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_constant__ KeyProductArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     KpShared &sh = *reinterpret_cast<KpShared *>(smem);
     uint8_t *table = smem + kHeader;
     uint8_t *stages = table + kp_table_bytes(a.N);
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const uint32_t N = a.N, groups = N / 8, n_chunks = N / kChunkWords;
+    const uint32_t N = a.N, groups = N / 8, n_chunks = kHalf ? 1 : N / kChunkWords;
     const uint32_t n_stages = kp_stages(N);
 
     if (threadIdx.x == 0) {
@@ -211,7 +213,7 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
                 const uint64_t r = r0 + h * (kRows / 2);
-                f_src[h] = f_item < a.items && r < a.n_rows
+                f_src[h] = f_item < a.items && r < a.n_rows && (!kHalf || l < groups)
                                ? reinterpret_cast<const uint32_t *>(kp_row(a, r)) + (N - 8 * (l + 1))
                                : nullptr;
             }
@@ -306,7 +308,7 @@ __global__ void __launch_bounds__(kKpThreads, 1) k_key_product(const __grid_cons
                 if (leader) {
                     if (w) {
 #pragma unroll
-                        for (uint32_t j = 0; j < kChunkWords / 16; ++j)
+                        for (uint32_t j = 0; j < (kHalf ? 2 : kChunkWords / 16); ++j)
                             umma_f16(d, da + j * (2 * kGroupBytes / 16), b + j * 16, idesc, c + j > 0 ? 1u : 0u);
                     }
                     umma_commit(&sh.a_empty[s]);
@@ -422,7 +424,7 @@ __global__ void k_clear_bodies(const __grid_constant__ KeyProductArgs a) {
 
 cudaError_t launch_key_product(KeyProductArgs a, int sm_count, cudaStream_t s) {
     if (a.n_rows == 0 || a.n_coef == 0) return cudaSuccess;
-    if (!key_product_supported(a.N) || a.N % kChunkWords || a.n_coef > a.N) return cudaErrorInvalidValue;
+    if (!key_product_supported(a.N) || (a.N & (a.N - 1)) || a.n_coef > a.N) return cudaErrorInvalidValue;
     const uint64_t row_tiles = (a.n_rows + kRows - 1) / kRows;
     const uint32_t coef_pad = (a.n_coef + 15u) & ~15u;
     // Pairs of column tiles per 32 rows: as few as the accumulators allow (a
@@ -437,7 +439,9 @@ cudaError_t launch_key_product(KeyProductArgs a, int sm_count, cudaStream_t s) {
     a.items = row_tiles * a.pairs;
     a.vec_rows = ((reinterpret_cast<uintptr_t>(a.rows) | a.stride) & 15u) == 0;
     a.vec_scores = ((reinterpret_cast<uintptr_t>(a.scores) | (uint64_t(a.n_coef) * 4)) & 7u) == 0;
-    auto *fn = a.scores ? k_key_product<true> : k_key_product<false>;
+    const bool half = a.N < kChunkWords;
+    auto *fn = a.scores ? (half ? k_key_product<true, true> : k_key_product<true, false>)
+                        : (half ? k_key_product<false, true> : k_key_product<false, false>);
     fn<<<uint32_t(std::min<uint64_t>(a.items, uint64_t(sm_count))), kKpThreads, kp_smem(a.N), s>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess && !a.scores)
@@ -446,7 +450,8 @@ cudaError_t launch_key_product(KeyProductArgs a, int sm_count, cudaStream_t s) {
 }
 
 cudaError_t configure_key_product() {
-    for (auto *fn : {k_key_product<true>, k_key_product<false>}) {
+    for (auto *fn : {k_key_product<true, false>, k_key_product<false, false>, k_key_product<true, true>,
+                     k_key_product<false, true>}) {
         const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    int(std::max(kp_smem(1024), kp_smem(kKeyMaxN))));
         if (e != cudaSuccess) return e;

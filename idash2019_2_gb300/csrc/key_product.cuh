@@ -19,7 +19,7 @@ struct KeyBits {
 bool key_bits(const int32_t *key, uint32_t N, KeyBits *out);
 
 // N the product kernel is built for (a power of two).
-inline bool key_product_supported(uint32_t N) { return N >= 64 && N <= kKeyMaxN; }
+inline bool key_product_supported(uint32_t N) { return N >= 32 && N <= kKeyMaxN; }
 
 struct KeyProductArgs {
     KeyBits key;

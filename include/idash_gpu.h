@@ -462,7 +462,7 @@ idash_status idash_encrypt_files(int device, const char *keys_file, const char *
  * d_out[r * num_samples + j] = float(phase_r[j] / 2^32).  key: the key's N
  * integer coefficients in host memory (binary for TFHE keys; any integers
  * are accepted).  N a power of two in [4, 2048].  Asynchronous on `stream`
- * once the key has been read: binary keys with N >= 64 travel in the launch
+ * once the key has been read: binary keys with N >= 32 travel in the launch
  * parameters, others are staged in device memory in stream order. */
 idash_status idash_decrypt_trlwe_device(idash_ctx *ctx, const int32_t *key, uint32_t N, const void *d_in,
                                         const idash_row_layout *in_layout, uint64_t n_rows, uint32_t num_samples,
