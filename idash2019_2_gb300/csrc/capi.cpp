@@ -54,6 +54,7 @@ struct Candidate {
     uint32_t w, g, slots, terms, groups, cps;
     uint32_t stages = 1;  // kWs: buffers in the ring
     bool split = false;   // plan neighbourhoods larger than a window as parts
+    bool spare = false;   // timed only where the tensor-core plan is not there
 };
 
 // Shared-memory carve-up of one buffer: a window-kernel CTA for `cps` CTAs
@@ -464,6 +465,13 @@ std::vector<Candidate> candidates(idash_model *m) {
             for (uint32_t stages : {2u, 3u})
                 if (window_limits(ctx, KernelKind::kWs, w, 1, &c, stages)) out.push_back(c);
     }
+    // Several regions to a row: the tensor-core plan was the fastest, or within 2%
+    // of it, for 19 of 22 shapes, and a window plan of 512 or 1,024 words for the
+    // others (few terms to an output).  With all of them timed, a new model's first
+    // pass took up to 4% longer than without the tensor-core plan.
+    if (m->form == Form::kTrlwe && m->tp.num_regions > 1 && !out.empty() && out[0].kind == KernelKind::kTc)
+        for (Candidate &c : out)
+            c.spare = c.kind != KernelKind::kTc && !(c.kind == KernelKind::kWindow && (c.w == 1024 || c.w == 512));
     // then the same shapes with split plans: used only when no shape fits
     // the model whole (the autotuner skips them once one has)
     if (ctx->opt_split) {
@@ -497,21 +505,24 @@ bool autotune_wanted(idash_model *m) { return !m->tuned && m->ctx->opt_kernel !=
 
 // Autotuning: the candidates' plans are built on host threads, one per
 // host core up to kPlanThreads at a time, then each is uploaded and timed in order by
-// time_fn (milliseconds per unit, <= 0 when it failed).  Split candidates
-// are tried only when no whole one worked.  The fastest becomes the model's
-// plan (or the first feasible one, when none could be timed).
+// time_fn (milliseconds per unit, <= 0 when it failed).  Spare candidates are
+// tried only where the tensor-core plan did not work, split ones only when no
+// whole one worked.  The fastest becomes the model's plan (or the first feasible
+// one, when none could be timed).
 constexpr size_t kPlanThreads = 16;
 
 template <typename TimeFn>
 idash_status autotune(idash_model *m, TimeFn time_fn) {
-    const std::vector<Candidate> cands = candidates(m);
+    std::vector<Candidate> cands = candidates(m);
+    auto rank = [](const Candidate &c) { return c.split ? 2 : c.spare ? 1 : 0; };
+    std::stable_sort(cands.begin(), cands.end(), [&](const Candidate &x, const Candidate &y) { return rank(x) < rank(y); });
     float best = -1.f;
     bool best_is_current = false;
     Candidate best_c{};
     BuiltPlan best_plan;
-    auto try_plan = [&](const Candidate &c, BuiltPlan &&b) {
+    auto try_plan = [&](const Candidate &c, BuiltPlan &&b) {  // whether it works
         best_is_current = false;
-        if (upload_plan(m, c, std::move(b)) != IDASH_OK) return;
+        if (upload_plan(m, c, std::move(b)) != IDASH_OK) return false;
         const float ms = time_fn();
         if (ms > 0 && (best < 0 || ms < best)) {
             best = ms;
@@ -519,44 +530,39 @@ idash_status autotune(idash_model *m, TimeFn time_fn) {
             best_c = c;
             best_plan.plan = std::move(m->plan);  // given back below, or the next upload replaces it
         }
+        return ms > 0;
     };
     // The tensor-core plan is the largest to upload and often the fastest: it
-    // is built with the first ones and timed last of the whole candidates, as
-    // what was timed last needs no second upload when it wins.
+    // is built with the first ones and timed last of them, as what was timed
+    // last needs no second upload when it wins.
     Candidate late_c{};
     BuiltPlan late;
-    bool have_late = false;
+    bool have_late = false, late_worked = false;
     auto try_late = [&]() {
-        if (have_late) try_plan(late_c, std::move(late));
+        if (have_late) late_worked = try_plan(late_c, std::move(late));
         have_late = false;
     };
-    bool stop = false;
     const size_t width = std::max<size_t>(1, std::min<size_t>(kPlanThreads, std::thread::hardware_concurrency()));
-    for (size_t i = 0; i < cands.size() && !stop; i += width) {
-        const size_t n = std::min(width, cands.size() - i);
-        // split candidates are seldom wanted: not built where a whole one is there
-        if (cands[i].split) {
-            try_late();
-            if (best >= 0) break;
-        }
+    size_t n = 0;
+    for (size_t i = 0; i < cands.size(); i += n) {
+        // batches of one rank
+        for (n = 1; n < width && i + n < cands.size() && rank(cands[i + n]) == rank(cands[i]); ++n) {}
+        if (rank(cands[i]) > 0) try_late();
+        if (rank(cands[i]) == 1 && late_worked) continue;
+        if (rank(cands[i]) == 2 && best >= 0) break;
         std::vector<BuiltPlan> built(n);
         std::vector<std::thread> threads;
         for (size_t k = 0; k < n; ++k)
             threads.emplace_back([&, k] { built[k] = make_plan(m, cands[i + k]); });
         for (auto &t : threads) t.join();
-        for (size_t k = 0; k < n && !stop; ++k) {
-            const Candidate &c = cands[i + k];
-            if (c.kind == KernelKind::kTc) {
-                late_c = c;
+        for (size_t k = 0; k < n; ++k) {
+            if (cands[i + k].kind == KernelKind::kTc) {
+                late_c = cands[i + k];
                 late = std::move(built[k]);
                 have_late = true;
-                continue;
+            } else {
+                try_plan(cands[i + k], std::move(built[k]));
             }
-            if (c.split) {
-                try_late();
-                stop = best >= 0;
-            }
-            if (!stop) try_plan(c, std::move(built[k]));
         }
     }
     try_late();
