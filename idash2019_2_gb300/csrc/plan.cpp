@@ -335,20 +335,6 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
     if (k_max < 16) return "no K satisfies the exactness bound";
 
     plan->tc_out.resize(n_out);
-    for (uint64_t o = 0; o < n_out; ++o) {
-        int64_t s0 = 0, s1 = 0;  // K's bound keeps 128 times each below 2^22
-        for (uint64_t t = nm.nptr[o]; t < nm.nptr[o + 1]; ++t) {
-            const uint32_t c = nm.ncoef[t];
-            const int32_t c0 = int32_t((c + 128u) & 255u) - 128;
-            s0 += c0;
-            s1 += c0 + (int64_t(int32_t(c)) - c0) / 256;
-        }
-        TcOut &x = plan->tc_out[o];
-        x.bias = nm.bias[o];
-        x.offset = 128u * uint32_t(s0) + 0x01010100u * 128u * uint32_t(s1);
-        x.m0 = 0.75f - float(128 * s0) * 0x1p-24f;
-        x.m1 = 0.75f - float(128 * s1) * 0x1p-24f;
-    }
     plan->phase_begin.push_back(0);
     std::vector<uint64_t> win, merged;
     uint64_t chunks = 0, scattered = 0;
@@ -401,6 +387,7 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         for (uint64_t p = o; p < e; ++p) {
             const uint32_t m = uint32_t(p - o);
             size_t idx = 0;
+            int64_t s0 = 0, s1 = 0;  // K's bound keeps 128 times each below 2^22
             for (uint64_t t = nm.nptr[p]; t < nm.nptr[p + 1]; ++t) {
                 while (win[idx] != nm.nkey[t]) ++idx;
                 const uint32_t c = nm.ncoef[t];
@@ -409,7 +396,14 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
                 const uint16_t h0 = half_bits(c0), h1 = half_bits(c1);
                 std::memcpy(A + tc_a_offset(m, uint32_t(idx)), &h0, 2);
                 std::memcpy(A + plane + tc_a_offset(m, uint32_t(idx)), &h1, 2);
+                s0 += c0;
+                s1 += c0 + c1;
             }
+            TcOut &x = plan->tc_out[p];
+            x.bias = nm.bias[p];
+            x.offset = 128u * uint32_t(s0) + 0x01010100u * 128u * uint32_t(s1);
+            x.m0 = 0.75f - float(128 * s0) * 0x1p-24f;
+            x.m1 = 0.75f - float(128 * s1) * 0x1p-24f;
         }
         plan->max_block_slots = std::max<uint32_t>(plan->max_block_slots, b.n_slots);
         plan->max_block_terms = std::max(plan->max_block_terms, k_pad);
@@ -417,9 +411,9 @@ std::string build_tc_plan(const PlanInput &in, const TcLimits &lim, Plan *plan, 
         o = e;
     }
     plan->tc_producers = 4 * scattered > chunks ? kTcMaxProducers : 1;
-    uint32_t rotations = 0;  // all of them, or-ed
-    for (uint64_t k : nm.nkey) rotations |= uint32_t(k);
     if (in.form == Form::kTrlwe && in.num_regions > 1) {
+        uint32_t rotations = 0;  // all of them, or-ed
+        for (uint64_t k : nm.nkey) rotations |= uint32_t(k);
         // a tile of columns is inside one polynomial, and a rotation a mask
         if (in.N % 64 != 0 || (in.N & (in.N - 1)) != 0) return "the tensor-core plan rotates rows of 2^k >= 64 coefficients";
         plan->tc_rot_bytes = rotations & 1u ? 4 : rotations & 2u ? 8 : 16;
