@@ -191,11 +191,14 @@ idash_status build_and_upload(idash_model *m, const Candidate &c) { return uploa
 // 3,000 targets, 10 neighbours 51.4 and 47.2 us; 200 targets, 20 neighbours
 // 14.5 and 12.6; 8,000 targets, 700 individuals 60.5 and 51.4.
 //
-// LWE rows are long: larger units write few neighbouring columns of many rows
-// at a time, and lose to memory what they save (37 individuals, n = 630: 0.240
-// ms with 6 slices a unit, 0.253 with 8, 0.277 with 16, 0.271 with 2; 100
-// individuals, 6,000 outputs: 0.632, 0.648, 0.659 and 0.685), so at most 6.
-// About 32 units a CTA where the digits are not loaded ahead (their load is
+// LWE rows are long, and cost more by far with fewer than 6 slices a unit; what
+// more than 6 do depends on whether every row starts on a 32-byte sector.  With 2,
+// 6, 8 and 16 slices, microseconds: 100 individuals, n = 1,024, 6,000 outputs, off
+// a sector 662, 637, 649, 653, on one 629, 547, 539, 529; 37 individuals, n = 630
+// 269, 243, 245, 260 and 257, 228, 227, 236; 300 individuals, n = 500 862, 800,
+// 804, 810 and 836, 754, 751, 754; 10 individuals, n = 1,024 297, 255, 254, 260 and
+// 286, 243, 240, 237.  At most 6: the best or within 1% of it off a sector, within
+// 4% on one.  About 32 units a CTA where the digits are not loaded ahead (their load is
 // then worth more slices: 5 to 50 neighbours 5.98 ms, 6.07 with 6 slices) and
 // for rows of several regions (their zeros come in bursts: 0.182 and 0.203).
 void tc_units(ScoreArgs *a, uint32_t ctas, double spread, bool digits_ahead) {

@@ -93,7 +93,7 @@ extern "C" idash_status idash_decrypt_trlwe_device(idash_ctx *ctx, const int32_t
     const uint8_t *in = static_cast<const uint8_t *>(d_in) + in_layout->payload_offset;
     // Binary keys (TFHE's) of a size the product kernel takes: tensor cores,
     // the key in the launch parameters.  242,646 rows x 1,000 scores at
-    // N = 1024: 6.90 ms with the product on CUDA cores, 0.95 ms here.
+    // N = 1024: 6.90 ms with the product on CUDA cores, 0.96 ms here.
     KeyProductArgs kp{};
     if (key_product_supported(N) && key_bits(key, N, &kp.key)) {
         kp.rows = const_cast<uint8_t *>(in);  // read only when scores are asked for

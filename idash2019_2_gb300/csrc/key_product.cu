@@ -38,7 +38,7 @@
 //              row's body words are in registers before the sums are ready.
 // Every wait is bounded and ends when another role raised the abort flag.
 //
-// What bounds it: 242,646 masks x 1,000 coefficients take 0.95 ms (6.90 ms as
+// What bounds it: 242,646 masks x 1,000 coefficients take 0.96 ms (6.90 ms as
 // sums over the key's set bits on CUDA cores; 1.64 ms with 40 rows a tile, the
 // digits exchanged by shuffles and one warp for both tiles' MMAs).  An item
 // (32 rows x 512 coefficients) takes 18,000 cycles, of which its MMAs are

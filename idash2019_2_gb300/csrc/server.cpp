@@ -28,7 +28,7 @@
 //               segment it holds: all queued behind the launch when it is
 //               issued, so that the host is in no step between scoring and
 //               completion (it was in three: one request of 10 targets took
-//               281 us, now 115; nine of 6 targets 491, now 266).  Copies to
+//               281 us, now 106; nine of 6 targets 419, now 267).  Copies to
 //               pageable memory would hold the thread up until the launch is
 //               done, so those are issued after it, on a stream of their own;
 //   completion  a copied segment's memory returns to the arena; a request
