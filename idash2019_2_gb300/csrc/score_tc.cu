@@ -524,6 +524,7 @@ __global__ void __launch_bounds__(tc_threads(kEpi, kConv, kConvWarps, kProducers
                         rr.next(a.tc_raw_stages);
                         continue;
                     }
+                    // undefined where lane c has given up: only a coordinate, which the map bounds
                     const int32_t r0 = int32_t(__shfl_sync(0xFFFFFFFFu, first, c));
                     uint64_t *full = &sh.raw_full[rr.s];
                     uint8_t *dst = raw + rr.s * kRawStageBytes;

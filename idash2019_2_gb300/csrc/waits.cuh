@@ -13,7 +13,8 @@ namespace idash {
 //   - leaves the loop, if nothing in it waits for the other lanes; or
 //   - exits (return), since a warp's barriers, shuffles and votes and the CTA's
 //     barriers are for the threads that have not exited (values from lanes that
-//     have are undefined: no address may depend on them).
+//     have are undefined: no address depends on them but by a tensor map, which
+//     bounds it).
 // (One verdict for all by a shuffle or vote after each wait: 0.2 to 2.6% of a
 // scoring pass with TRLWE rows, 1.5 to 5% with LWE rows.)
 __device__ __forceinline__ bool tc_wait(uint32_t *abort, uint64_t *bar, uint32_t parity, uint32_t *err,
